@@ -197,6 +197,36 @@ def test_filtered_probabilities_match_oracle_bit_for_bit(vocab, dtype, levels):
     assert torch.equal(plain.cpu(), _oracle_probabilities(logits, temperature, [-1] * rows, [1.0] * rows))
 
 
+@pytest.mark.parametrize("vocab,first,dtype", [(49152, 0, torch.float32), (50257, 0, torch.float32), (8191, 3, torch.bfloat16),
+                                               (2049, 1, torch.float32), (513, 0, torch.float16), (40, 0, torch.float32)])
+def test_filters_where_a_selection_changes_its_way_match_oracle_bit_for_bit(vocab, first, dtype):
+    """top-k around a token per thread, candidates that fit and that do not, rows that are all ties, that have fewer finite logits than k,
+    that are flat or have one token; extreme temperatures; rows at any alignment."""
+    g = torch.Generator().manual_seed(vocab)
+    wide = torch.randn(16, first + vocab, generator=g) * 3
+    wide[1], wide[9] = 1.5, -0.0
+    wide[2, first + 30:] = float("-inf")
+    wide[3] *= 1e-3
+    wide[4, first + vocab // 2] = 1e4
+    wide[5] *= 3e3                # 3 * 3000 * 5 standard deviations < 65504, the largest float16
+    wide[6] -= 1e4
+    wide[13, first + vocab // 3:] = 2.0
+    wide = wide.to(dtype)
+    logits = wide[:, first:]
+    temperature = torch.tensor([0.8, 1.0, 0.7, 1.0, 0.5, 1.0, 1.0, 1e-3, 1e4, 1.0, 0.8, 0.8, 0.8, 0.8, 1.3, 1.3])
+    some = [50, 511, 512, 513, 1023, 1024, 1025, 3000, 1, 20, -1]
+    for shift in range(len(some)):
+        top_k = torch.tensor([some[(r + shift) % len(some)] for r in range(16)], dtype=torch.int32)
+        top_p = torch.tensor([[0.95, 1.0, 0.5, 1e-7, 0.9999][(r + 2 * shift) % 5] for r in range(16)])
+        want = _oracle_probabilities(logits.contiguous(), temperature, top_k, top_p)
+        got, status = rlt.probabilities(wide.cuda()[:, first:], temperature.cuda(), top_k.cuda(), top_p.cuda())
+        assert not status.any()
+        assert torch.equal(got.cpu(), want), (shift, [r for r in range(16) if not torch.equal(got[r].cpu(), want[r])])
+        uniforms = torch.rand(16, generator=g)
+        tokens, _ = rlt.sample_rows(wide.cuda()[:, first:], temperature.cuda(), uniforms.cuda(), top_k.cuda(), top_p.cuda())
+        assert torch.equal(tokens.cpu(), oracle.sample_rows(logits.contiguous(), temperature, uniforms, top_k, top_p)[0])
+
+
 def test_probabilities_reject_greedy_and_bad_rows():
     logits = torch.randn(3, 64)
     logits[2, 5] = float("nan")

@@ -75,8 +75,7 @@ __device__ __forceinline__ unsigned long long block_sum(unsigned long long v, un
 // Packed (value, lowest index) maximum of one row by the whole CTA.  16-byte loads when the row
 // allows them, four in flight per thread (a row is only a few hundred KB: latency, not issue
 // rate, decides how fast one CTA can stream it).
-// kPlain: `row` may point to shared memory (a staged row), so no global-only load forms.
-template <typename T, int kThreads, bool kPlain = false>
+template <typename T, int kThreads>
 __device__ __forceinline__ unsigned long long block_max_key(const T* __restrict__ row, int vocab,
                                                            unsigned long long* scratch) {
   constexpr int kVec = 16 / sizeof(T);
@@ -90,7 +89,7 @@ __device__ __forceinline__ unsigned long long block_max_key(const T* __restrict_
 #pragma unroll
       for (int k = 0; k < kDepth; ++k) {
         const int i = base + k * kThreads;
-        if (i < nvec) raw[k] = kPlain ? rv[i] : __ldcs(rv + i);
+        if (i < nvec) raw[k] = __ldcs(rv + i);
       }
 #pragma unroll
       for (int k = 0; k < kDepth; ++k) {
@@ -189,55 +188,58 @@ __device__ __forceinline__ float scaled_logit(const T* row, int v, float tempera
   return RLT_DIV(Elem<T>::to_float(row[v]), temperature);
 }
 
-// max of row / temperature.  Division by a positive temperature is monotonic, so
-// max_v (x_v / T) == (max_v x_v) / T exactly: the pass is a plain maximum over the raw logits
-// (NaN counts as the maximum and is then reported), one division at the end.
-template <typename T, int kThreads, bool kPlain = false>
-__device__ __forceinline__ RowNorm block_row_max(const T* __restrict__ row, int vocab, float temperature,
-                                                 unsigned long long* scratch) {
-  const unsigned long long best = block_max_key<T, kThreads, kPlain>(row, vocab, scratch);
-  RowNorm n;
-  uint32_t bits = static_cast<uint32_t>(best >> 32);
-  bits = (bits & 0x80000000u) ? (bits & 0x7fffffffu) : ~bits;
-  const float raw_max = __uint_as_float(bits);
-  n.m = RLT_DIV(raw_max, temperature);
-  n.ok = best != 0ull && raw_max == raw_max && n.m != INFINITY && n.m != -INFINITY;
-  n.z = 0.0f;
-  n.cut = whole_row();
-  return n;
-}
-
-// Normaliser of softmax(row / temperature) over the whole row.
-template <typename T, int kThreads, bool kPlain = false>
-__device__ __forceinline__ float block_full_sum(const T* __restrict__ row, int vocab, float temperature, float m,
-                                                unsigned long long* scratch) {
-  unsigned long long zfix = 0ull;
+// f(value, index) for every element of the row by the whole CTA, in no particular order: 16-byte loads, kDepth in flight per
+// thread, where the row allows them.  A row is a few hundred KB: the first pass over it reads HBM, the others L2.
+template <typename T, int kThreads, int kDepth = 4, typename F>
+__device__ __forceinline__ void for_row(const T* __restrict__ row, int vocab, F f) {
   constexpr int kVec = 16 / sizeof(T);
-  if ((reinterpret_cast<uintptr_t>(row) & 15u) == 0 && vocab % kVec == 0) {
+  int done = 0;
+  if ((reinterpret_cast<uintptr_t>(row) & 15u) == 0) {
     const uint4* rv = reinterpret_cast<const uint4*>(row);
     const int nvec = vocab / kVec;
-    for (int base = threadIdx.x; base < nvec; base += kThreads * 2) {
-      uint4 raw[2];
+    for (int base = threadIdx.x; base < nvec; base += kThreads * kDepth) {
+      uint4 raw[kDepth];
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
-        const int i = base + k * kThreads;
-        if (i < nvec) raw[k] = kPlain ? rv[i] : __ldg(rv + i);
-      }
+      for (int k = 0; k < kDepth; ++k)
+        if (base + k * kThreads < nvec) raw[k] = __ldg(rv + base + k * kThreads);
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
+      for (int k = 0; k < kDepth; ++k) {
         const int i = base + k * kThreads;
         if (i < nvec) {
           const T* e = reinterpret_cast<const T*>(&raw[k]);
 #pragma unroll
-          for (int j = 0; j < kVec; ++j)
-            zfix += rlt_fix_weight(rlt_expf(RLT_SUB(RLT_DIV(Elem<T>::to_float(e[j]), temperature), m)));
+          for (int j = 0; j < kVec; ++j) f(Elem<T>::to_float(e[j]), i * kVec + j);
         }
       }
     }
-  } else {
-    for (int v = threadIdx.x; v < vocab; v += kThreads)
-      zfix += rlt_fix_weight(rlt_expf(RLT_SUB(scaled_logit(row, v, temperature), m)));
+    done = nvec * kVec;
   }
+  for (int v = done + static_cast<int>(threadIdx.x); v < vocab; v += kThreads) f(Elem<T>::to_float(row[v]), v);
+}
+
+// A raw value below which no logit can have a scaled value >= t (rounding of the division and of this product included):
+// most tokens are outside a support and are dismissed by one comparison.
+__device__ __forceinline__ float raw_floor(float t, float temperature) {
+  const float x = t * temperature;
+  const float floor = x - (fabsf(x) * 0x1p-20f + temperature * 0x1p-140f + 0x1p-120f);
+  return floor == floor ? floor : -INFINITY;           // an infinite product says nothing
+}
+__device__ __forceinline__ float key_value(uint32_t key) {
+  return __uint_as_float((key & 0x80000000u) ? (key & 0x7fffffffu) : ~key);
+}
+// The same for the tokens of a cut; -inf where everything belongs to it.
+__device__ __forceinline__ float cut_floor(Cut cut, float temperature) {
+  return cut.key == 0u ? -INFINITY : raw_floor(key_value(cut.key), temperature);
+}
+
+// Normaliser of softmax(row / temperature) over the whole row.
+template <typename T, int kThreads>
+__device__ __forceinline__ float block_full_sum(const T* __restrict__ row, int vocab, float temperature, float m,
+                                                unsigned long long* scratch) {
+  unsigned long long zfix = 0ull;
+  for_row<T, kThreads, 2>(row, vocab, [&](float x, int) {
+    zfix += rlt_fix_weight(rlt_expf(RLT_SUB(RLT_DIV(x, temperature), m)));
+  });
   return rlt_fix_to_float(block_sum<kThreads>(zfix, scratch));
 }
 
@@ -246,30 +248,96 @@ template <typename T, int kThreads>
 __device__ __forceinline__ float block_cut_sum(const T* __restrict__ row, int vocab, float temperature, float m,
                                                Cut cut, unsigned long long* scratch) {
   unsigned long long zfix = 0ull;
-  for (int v = threadIdx.x; v < vocab; v += kThreads) {
-    const float t = scaled_logit(row, v, temperature);
-    if (rlt_in_support(rlt_order_key(t), v, cut.key, cut.limit)) zfix += rlt_fix_weight(rlt_expf(RLT_SUB(t, m)));
-  }
+  const float floor = cut_floor(cut, temperature);
+  for_row<T, kThreads>(row, vocab, [&](float x, int v) {
+    if (x >= floor) {
+      const float t = RLT_DIV(x, temperature);
+      if (rlt_in_support(rlt_order_key(t), v, cut.key, cut.limit)) zfix += rlt_fix_weight(rlt_expf(RLT_SUB(t, m)));
+    }
+  });
   return rlt_fix_to_float(block_sum<kThreads>(zfix, scratch));
 }
 
-// ---- top-k / top-p: radix select over the ranking ------------------------------------------
+// ---- top-k / top-p: selection over the ranking ----------------------------------------------
 // Both filters keep the ranks whose exclusive prefix WEIGHT is <= a limit: weight 1 per token
 // and limit k - 1 for top-k, the fixed-point probability mass and rlt_top_p_limit for top-p.
-// The cut is found digit by digit (four 8-bit digits of the order key, most significant first):
-// a histogram of weight per digit over the tokens that match the digits chosen so far, then the
-// digit in which the running weight, accumulated from the top, first exceeds the limit.  Equal
-// keys have equal weights, so inside the final tie group the kept count follows by division and
-// the cut index is the n-th matching token in index order.  A row is a few hundred KB and stays
-// in L2 between the passes.
+// Integer weights make the cut independent of how it is found.  Three ways, all over the row where it lies (L2 after the first
+// pass), several CTAs per SM:
+//   candidates   top-k up to a token per thread: at least k tokens reach the k-th largest of the threads' own maxima, so the few
+//                tokens at or above that value (70 for k = 50 of 49 152) hold the whole answer, and top-p inside it.
+//   buckets      every other filter: a histogram of weight over m - t in steps of 1/64 finds the step in which the running weight
+//                first exceeds the limit; its tokens are the candidates.
+//   digits       rows whose candidates do not fit (mass ties): a radix select over four 8-bit digits of the order key.
+// 128 requests of 5 rows of 49 152 fp32 logits, half of them with top-k 50 and top-p 0.95: the digits alone, over a row copied
+// to shared memory by one CTA per SM, took 595 us; this takes 141 us.
+constexpr int kCandidates = 2048;
+constexpr int kBuckets = 2048;
+
 struct SelectScratch {
-  unsigned long long mass[256];
-  unsigned int count[256];
+  union {
+    struct {                                // candidates, and the digits' histogram
+      unsigned long long weight[kCandidates];
+      uint32_t key[kCandidates];
+      int index[kCandidates];
+    };
+    unsigned long long bucket[kBuckets];
+    struct {
+      unsigned long long mass[256];
+      unsigned int count[256];
+    };
+  };
   unsigned long long above;
   int digit;
   int found;
+  int listed;
   int warp_counts[32];
 };
+
+__device__ __forceinline__ int bucket_of(float t, float m) {
+  const float d = RLT_SUB(m, t);
+  return d < 31.0f ? max(static_cast<int>(d * 64.0f), 0) : kBuckets - 1;
+}
+
+// Adds a token to the candidates; those that do not fit are only counted.
+__device__ __forceinline__ void list_token(SelectScratch& h, uint32_t key, int index) {
+  const int at = atomicAdd(&h.listed, 1);
+  if (at < kCandidates) { h.key[at] = key; h.index[at] = index; }
+}
+
+// The cut among n listed candidates with their weights, `above` being the weight of the tokens ranked before all of them.
+// A candidate whose weight no longer counts has weight 0 and key 0.  The running weight must exceed the limit inside the list.
+template <int kThreads>
+__device__ __forceinline__ Cut list_select(SelectScratch& h, int n, unsigned long long above, unsigned long long limit, Cut outer,
+                                           unsigned long long* scratch) {
+  auto weight_where = [&](auto&& counts) {
+    unsigned long long sum = 0ull;
+    for (int j = threadIdx.x; j < n; j += kThreads)
+      if (counts(j)) sum += h.weight[j];
+    return block_sum<kThreads>(sum, scratch);
+  };
+  uint32_t key = 0u;                        // the largest key for which the weight of all tokens from it on exceeds the limit
+  for (int bit = 31; bit >= 0; --bit) {
+    const uint32_t next = key | (1u << bit);
+    if (above + weight_where([&](int j) { return h.key[j] >= next; }) > limit) key = next;
+  }
+  const unsigned long long before = above + weight_where([&](int j) { return h.key[j] > key; });
+  int ties = 0;
+  unsigned long long each = 0ull;
+  for (int j = threadIdx.x; j < n; j += kThreads)
+    if (h.key[j] == key) { ++ties; each = h.weight[j]; }
+  ties = static_cast<int>(block_sum<kThreads>(static_cast<unsigned long long>(ties), scratch));
+  each = block_max<kThreads>(each, scratch);
+  const unsigned long long keep = (limit - before) / each + 1ull;
+  if (keep >= static_cast<unsigned long long>(ties)) return Cut{key, key == outer.key ? outer.limit : 0x7fffffff};
+  int index = 0;                            // the largest index with fewer than `keep` of the tied tokens before it
+  for (int bit = 30; bit >= 0; --bit) {
+    const int next = index | (1 << bit);
+    unsigned long long count = 0ull;
+    for (int j = threadIdx.x; j < n; j += kThreads) count += h.key[j] == key && h.index[j] < next;
+    if (block_sum<kThreads>(count, scratch) < keep) index = next;
+  }
+  return Cut{key, index};
+}
 
 // One shared-memory atomic per distinct digit in the warp: lanes with the same digit find each
 // other with match.any and add their weights with two integer warp reductions (a weight is below
@@ -388,41 +456,152 @@ __device__ __forceinline__ Cut block_select(const T* __restrict__ row, int vocab
                                                   static_cast<unsigned int>(keep), h)};
 }
 
+// The cut by buckets (digits where the bucket's tokens do not fit the list); `inv` is 1 / z.
+template <typename T, int kThreads, bool kByMass>
+__device__ __forceinline__ Cut bucket_select(const T* __restrict__ row, int vocab, float temperature, float m, float inv, Cut outer,
+                                             unsigned long long limit, unsigned long long* scratch, SelectScratch& h) {
+  constexpr int kOwn = kBuckets / kThreads;
+  const float floor = cut_floor(outer, temperature);
+  const auto weight = [&](float t) { return kByMass ? rlt_fix_weight(rlt_draw_mass(rlt_expf(RLT_SUB(t, m)), inv)) : 1ull; };
+  __syncthreads();
+  for (int i = threadIdx.x; i < kBuckets; i += kThreads) h.bucket[i] = 0ull;
+  if (threadIdx.x == 0) { h.digit = -1; h.listed = 0; }
+  __syncthreads();
+  for_row<T, kThreads, 2>(row, vocab, [&](float x, int v) {
+    if (x >= floor) {
+      const float t = RLT_DIV(x, temperature);
+      if (rlt_in_support(rlt_order_key(t), v, outer.key, outer.limit)) {
+        const unsigned long long w = weight(t);
+        if (w != 0ull) atomicAdd(&h.bucket[bucket_of(t, m)], w);
+      }
+    }
+  });
+  __syncthreads();
+  // thread i scans buckets kOwn * i ..
+  unsigned long long own[kOwn], local = 0ull;
+#pragma unroll
+  for (int j = 0; j < kOwn; ++j) { own[j] = h.bucket[kOwn * threadIdx.x + j]; local += own[j]; }
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  unsigned long long before = local;
+#pragma unroll
+  for (int x = 1; x < 32; x <<= 1) {
+    const unsigned long long o = __shfl_up_sync(0xffffffffu, before, x);
+    if (lane >= x) before += o;
+  }
+  if (lane == 31) scratch[warp] = before;
+  __syncthreads();
+  before -= local;
+  for (int w = 0; w < warp; ++w) before += scratch[w];
+  if (before <= limit && before + local > limit) {      // one thread at most
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) {
+      if (h.digit < 0) {
+        if (before + own[j] > limit) { h.digit = kOwn * threadIdx.x + j; h.above = before; }
+        before += own[j];
+      }
+    }
+  }
+  __syncthreads();
+  const int crossing = h.digit;
+  const unsigned long long above = h.above;
+  if (crossing < 0) return outer;           // everything stays
+  for_row<T, kThreads>(row, vocab, [&](float x, int v) {
+    if (x >= floor) {
+      const float t = RLT_DIV(x, temperature);
+      const uint32_t key = rlt_order_key(t);
+      if (bucket_of(t, m) == crossing && rlt_in_support(key, v, outer.key, outer.limit)) list_token(h, key, v);
+    }
+  });
+  __syncthreads();
+  const int n = h.listed;
+  if (n > kCandidates) return block_select<T, kThreads, kByMass>(row, vocab, temperature, m, inv, outer, limit, h);
+  for (int j = threadIdx.x; j < n; j += kThreads) h.weight[j] = weight(key_value(h.key[j]));
+  return list_select<kThreads>(h, n, above, limit, outer, scratch);
+}
+
 // max, support and normaliser of the distribution Sampler.probabilities builds for one row
 // (vllm_rlt/worker/sampler.py:37-55): softmax(row / T) restricted to top-k, then to top-p.
 // top_k <= 0 or >= vocab and top_p >= 1 switch the filters off.
-template <typename T, int kThreads, bool kPlain = false>
+// Division by a positive temperature is monotonic, so max_v (x_v / T) == (max_v x_v) / T exactly: the first pass is a plain
+// maximum over the raw logits, one division at the end.
+template <typename T, int kThreads>
 __device__ __forceinline__ RowNorm block_normalise(const T* __restrict__ row, int vocab, float temperature,
                                                    int top_k, float top_p, unsigned long long* scratch,
                                                    SelectScratch& h) {
-  RowNorm n = block_row_max<T, kThreads, kPlain>(row, vocab, temperature, scratch);
-  if (!n.ok) return n;
   const bool use_k = top_k > 0 && top_k < vocab, use_p = top_p < 1.0f;
+  float own = -INFINITY;
+  bool nan = false;
+  for_row<T, kThreads>(row, vocab, [&](float x, int) {
+    own = fmaxf(own, x);
+    nan |= x != x;
+  });
+  const uint32_t own_key = rlt_order_key(own);
+  const uint32_t top = __reduce_max_sync(0xffffffffu, nan ? 0xffffffffu : own_key);
+  RowNorm n;
+  const uint32_t best = static_cast<uint32_t>(block_max<kThreads>(top, scratch));
+  n.m = best == 0xffffffffu ? NAN : RLT_DIV(key_value(best), temperature);
+  n.ok = n.m == n.m && n.m != INFINITY && n.m != -INFINITY;
+  n.z = 0.0f;
+  n.cut = whole_row();
+  if (!n.ok) return n;
+  const unsigned long long limit_p = rlt_top_p_limit(top_p);
   if (use_k) {
-    n.cut = block_select<T, kThreads, false>(row, vocab, temperature, n.m, 0.0f, whole_row(),
-                                             static_cast<unsigned long long>(top_k - 1), h);
+    int listed = kCandidates + 1;
+    if (top_k <= kThreads) {
+      uint32_t reached = 0u;                // at least top_k of the threads' maxima, in 18 bits
+      for (int bit = 31; bit >= 14; --bit)
+        if (__syncthreads_count(own_key >= (reached | (1u << bit))) >= top_k) reached |= 1u << bit;
+      // (keys below that of the lowest finite value come from threads without one)
+      const float floor = reached < 0x00800000u ? -INFINITY : raw_floor(RLT_DIV(key_value(reached), temperature), temperature);
+      if (threadIdx.x == 0) h.listed = 0;
+      __syncthreads();
+      for_row<T, kThreads>(row, vocab, [&](float x, int v) {
+        if (x >= floor) list_token(h, rlt_order_key(RLT_DIV(x, temperature)), v);
+      });
+      __syncthreads();
+      listed = h.listed;
+    }
+    if (listed <= kCandidates) {
+      for (int j = threadIdx.x; j < listed; j += kThreads) h.weight[j] = 1ull;
+      n.cut = list_select<kThreads>(h, listed, 0ull, static_cast<unsigned long long>(top_k - 1), whole_row(), scratch);
+      const auto sum_kept = [&]() {
+        unsigned long long zfix = 0ull;
+        for (int j = threadIdx.x; j < listed; j += kThreads)
+          if (rlt_in_support(h.key[j], h.index[j], n.cut.key, n.cut.limit)) zfix += rlt_fix_weight(rlt_expf(RLT_SUB(key_value(h.key[j]), n.m)));
+        return rlt_fix_to_float(block_sum<kThreads>(zfix, scratch));
+      };
+      n.z = sum_kept();
+      if (use_p) {
+        const Cut outer = n.cut;
+        const float inv = RLT_DIV(1.0f, n.z);
+        unsigned long long mass = 0ull;
+        for (int j = threadIdx.x; j < listed; j += kThreads) {
+          unsigned long long w = 0ull;
+          if (rlt_in_support(h.key[j], h.index[j], outer.key, outer.limit)) w = rlt_fix_weight(rlt_draw_mass(rlt_expf(RLT_SUB(key_value(h.key[j]), n.m)), inv));
+          else h.key[j] = 0u;
+          h.weight[j] = w;
+          mass += w;
+        }
+        if (block_sum<kThreads>(mass, scratch) > limit_p) {
+          n.cut = list_select<kThreads>(h, listed, 0ull, limit_p, outer, scratch);
+          n.z = sum_kept();
+        }
+      }
+      return n;
+    }
+    n.cut = bucket_select<T, kThreads, false>(row, vocab, temperature, n.m, 0.0f, whole_row(),
+                                              static_cast<unsigned long long>(top_k - 1), scratch, h);
     n.z = block_cut_sum<T, kThreads>(row, vocab, temperature, n.m, n.cut, scratch);
   } else {
-    n.z = block_full_sum<T, kThreads, kPlain>(row, vocab, temperature, n.m, scratch);
+    n.z = block_full_sum<T, kThreads>(row, vocab, temperature, n.m, scratch);
   }
   if (use_p) {
     const Cut outer = n.cut;
-    n.cut = block_select<T, kThreads, true>(row, vocab, temperature, n.m, RLT_DIV(1.0f, n.z), outer,
-                                            rlt_top_p_limit(top_p), h);
+    n.cut = bucket_select<T, kThreads, true>(row, vocab, temperature, n.m, RLT_DIV(1.0f, n.z), outer, limit_p, scratch, h);
     if (n.cut.key != outer.key || n.cut.limit != outer.limit)
       n.z = block_cut_sum<T, kThreads>(row, vocab, temperature, n.m, n.cut, scratch);
   }
   return n;
-}
-
-// A row copied to shared memory as fp32 (exact for all three storage types).  The filters make a
-// dozen passes over a row; from shared memory a pass costs a few microseconds instead of one L2
-// round trip per element and thread.  Used when the caller passes filters and the row fits.
-template <typename T, int kThreads>
-__device__ __forceinline__ const float* stage_row(const T* __restrict__ row, int vocab, float* staged) {
-  for (int v = threadIdx.x; v < vocab; v += kThreads) staged[v] = Elem<T>::to_float(row[v]);
-  __syncthreads();
-  return staged;
 }
 
 // exp(t_v - max) for a token of the support, 0 outside it.
@@ -438,55 +617,84 @@ __device__ __forceinline__ float prob_at(const T* row, int v, float temperature,
   return RLT_DIV(exp_at(row, v, temperature, n), n.z);
 }
 
-// Fixed-point draw weight of token v: p[v] (plain) or max(p[v] - q[v], 0) (residual), in the
-// division-free form of rlt_canonical.h; `inv` is 1/zp or 1/(zp*zq).
-template <typename T>
-__device__ __forceinline__ unsigned long long draw_weight(const T* prow, const RowNorm& pn, const T* qrow,
-                                                          const RowNorm& qn, bool residual, int v,
-                                                          float temperature, float inv) {
-  const float ep = exp_at(prow, v, temperature, pn);
-  if (!residual) return rlt_fix_weight(rlt_draw_mass(ep, inv));
-  return rlt_fix_weight(rlt_residual_mass(ep, exp_at(qrow, v, temperature, qn), pn.z, qn.z, inv));
-}
-
-// Inverse-CDF draw over fixed-point weights in ascending token index; -1 if the mass is zero.
-// Thread t owns the contiguous tokens [t*span, (t+1)*span); its weights stay in registers
-// between the sum and the search when the span is small enough.
+// Inverse-CDF draw over fixed-point weights in ascending token index, p[v] (plain) or max(p[v] - q[v], 0) (residual) in the
+// division-free form of rlt_canonical.h; -1 if the mass is zero.  A warp owns a run of tokens and reads it 128 tokens at a time, four
+// per lane; the warp in whose run the threshold falls goes over its run once more.  Tokens outside p's support weigh nothing and are
+// dismissed by one comparison, q is read where p has mass only.  (A run of tokens per THREAD, the earlier split, read a line per
+// lane: a residual draw from two rows of 49 152 took 74 us, this 56.)
 template <typename T, int kThreads>
 __device__ __forceinline__ int block_draw(const T* __restrict__ prow, const RowNorm& pn,
                                           const T* __restrict__ qrow, const RowNorm& qn, bool residual,
                                           int vocab, float temperature, float u, unsigned long long* scratch,
                                           int* token_slot) {
+  constexpr int kWarps = kThreads / 32, kLane = 4, kStep = 32 * kLane;
+  struct __align__(kLane * sizeof(T)) Four { T e[kLane]; };
   const float inv = residual ? RLT_DIV(1.0f, RLT_MUL(pn.z, qn.z)) : RLT_DIV(1.0f, pn.z);
-  const int span = (vocab + kThreads - 1) / kThreads;
-  const int begin = min(static_cast<int>(threadIdx.x) * span, vocab), end = min(begin + span, vocab);
-  unsigned long long local = 0ull;
-  for (int v = begin; v < end; ++v) local += draw_weight(prow, pn, qrow, qn, residual, v, temperature, inv);
-  // exclusive scan over threads: inclusive warp scan, then warp totals
+  const float floor = cut_floor(pn.cut, temperature);
+  const bool vectors = (reinterpret_cast<uintptr_t>(prow) & (sizeof(Four) - 1)) == 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long inc = local;
+  const int run = (vocab + kWarps * kStep - 1) / (kWarps * kStep) * kStep;
+  const int begin = min(warp * run, vocab), end = min(begin + run, vocab);
+  const auto weigh = [&](int v, unsigned long long (&w)[kLane]) {      // tokens v .. v + 3
+    float x[kLane];
+    if (vectors && v + kLane <= end) {
+      const Four raw = *reinterpret_cast<const Four*>(prow + v);
 #pragma unroll
-  for (int x = 1; x < 32; x <<= 1) {
-    const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, x);
-    if (lane >= x) inc += o;
-  }
+      for (int j = 0; j < kLane; ++j) x[j] = Elem<T>::to_float(raw.e[j]);
+    } else {
+#pragma unroll
+      for (int j = 0; j < kLane; ++j) x[j] = v + j < end ? Elem<T>::to_float(prow[v + j]) : -INFINITY;
+    }
+    unsigned long long sum = 0ull;
+#pragma unroll
+    for (int j = 0; j < kLane; ++j) {
+      w[j] = 0ull;
+      if (v + j < end && x[j] >= floor) {
+        const float t = RLT_DIV(x[j], temperature);
+        if (rlt_in_support(rlt_order_key(t), v + j, pn.cut.key, pn.cut.limit)) {
+          const float e = rlt_expf(RLT_SUB(t, pn.m));
+          w[j] = rlt_fix_weight(residual ? rlt_residual_mass(e, exp_at(qrow, v + j, temperature, qn), pn.z, qn.z, inv) : rlt_draw_mass(e, inv));
+        }
+      }
+      sum += w[j];
+    }
+    return sum;
+  };
+  unsigned long long w[kLane], local = 0ull;
+#pragma unroll 2
+  for (int v = begin + lane * kLane; v < end; v += kStep) local += weigh(v, w);
+  local = warp_sum(local);
   __syncthreads();
-  if (lane == 31) scratch[warp] = inc;
+  if (lane == 0) scratch[warp] = local;
   if (threadIdx.x == 0) *token_slot = -1;
   __syncthreads();
   unsigned long long before = 0ull, total = 0ull;
-  for (int w = 0; w < kThreads / 32; ++w) {
-    const unsigned long long s = scratch[w];
-    if (w < warp) before += s;
+  for (int i = 0; i < kWarps; ++i) {
+    const unsigned long long s = scratch[i];
+    if (i < warp) before += s;
     total += s;
   }
   if (total != 0ull) {
     const unsigned long long threshold = rlt_draw_threshold(u, total);
-    unsigned long long prefix = before + inc - local;
-    if (prefix <= threshold && threshold < prefix + local) {
-      for (int v = begin; v < end; ++v) {
-        prefix += draw_weight(prow, pn, qrow, qn, residual, v, temperature, inv);
-        if (prefix > threshold) { *token_slot = v; break; }
+    if (before <= threshold && threshold < before + local) {           // one warp
+      for (int at = begin; at < end; at += kStep) {
+        const unsigned long long sum = weigh(at + lane * kLane, w);
+        unsigned long long upto = sum;
+#pragma unroll
+        for (int x = 1; x < 32; x <<= 1) {
+          const unsigned long long o = __shfl_up_sync(0xffffffffu, upto, x);
+          if (lane >= x) upto += o;
+        }
+        unsigned long long prefix = before + upto - sum;
+        if (prefix <= threshold && threshold < prefix + sum) {
+#pragma unroll
+          for (int j = 0; j < kLane; ++j) {
+            if (prefix <= threshold && threshold < prefix + w[j]) *token_slot = at + lane * kLane + j;
+            prefix += w[j];
+          }
+        }
+        before += __shfl_sync(0xffffffffu, upto, 31);
+        if (before > threshold) break;
       }
     }
   }
@@ -494,7 +702,7 @@ __device__ __forceinline__ int block_draw(const T* __restrict__ prow, const RowN
   return *token_slot;
 }
 
-template <typename T, bool kStaged>
+template <typename T>
 __global__ void __launch_bounds__(kSampleThreads)
 sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int vocab,
                    const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
@@ -510,17 +718,6 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int vocab,
   int token = -1;
   if (temp == 0.0f) {
     token = block_argmax<T, kSampleThreads>(row, vocab, scratch);
-  } else if constexpr (kStaged) {
-    extern __shared__ __align__(16) float staged[];
-    const float* frow = stage_row<T, kSampleThreads>(row, vocab, staged);
-    const RowNorm n = block_normalise<float, kSampleThreads, true>(frow, vocab, temp, top_k ? top_k[r] : -1,
-                                                                   top_p ? top_p[r] : 1.0f, scratch, select);
-    if (!n.ok) {
-      st = RLT_ROW_BAD_LOGITS;
-    } else {
-      token = block_draw<float, kSampleThreads>(frow, n, frow, n, false, vocab, temp, uniforms[r], scratch, &token_slot);
-      if (token < 0) st = RLT_ROW_INVALID_RESIDUAL;
-    }
   } else {
     const RowNorm n = block_normalise<T, kSampleThreads>(row, vocab, temp, top_k ? top_k[r] : -1,
                                                          top_p ? top_p[r] : 1.0f, scratch, select);
@@ -535,7 +732,7 @@ sample_rows_kernel(const T* __restrict__ logits, int64_t row_stride, int vocab,
 }
 
 // Sampler.probabilities for every row: fp32 [rows, vocab], zero outside the support.
-template <typename T, bool kStaged>
+template <typename T>
 __global__ void __launch_bounds__(kSampleThreads)
 probabilities_kernel(const T* __restrict__ logits, int64_t row_stride, int vocab,
                      const float* __restrict__ temperature, const int32_t* __restrict__ top_k,
@@ -548,19 +745,10 @@ probabilities_kernel(const T* __restrict__ logits, int64_t row_stride, int vocab
   const float temp = temperature[r];
   RowNorm n;
   n.ok = 0;
-  if constexpr (kStaged) {
-    extern __shared__ __align__(16) float staged[];
-    const float* frow = stage_row<T, kSampleThreads>(row, vocab, staged);
-    if (temp > 0.0f)
-      n = block_normalise<float, kSampleThreads, true>(frow, vocab, temp, top_k ? top_k[r] : -1,
-                                                       top_p ? top_p[r] : 1.0f, scratch, select);
-    for (int v = threadIdx.x; v < vocab; v += kSampleThreads) out[v] = n.ok ? prob_at(frow, v, temp, n) : 0.0f;
-  } else {
-    if (temp > 0.0f)
-      n = block_normalise<T, kSampleThreads>(row, vocab, temp, top_k ? top_k[r] : -1, top_p ? top_p[r] : 1.0f,
-                                             scratch, select);
-    for (int v = threadIdx.x; v < vocab; v += kSampleThreads) out[v] = n.ok ? prob_at(row, v, temp, n) : 0.0f;
-  }
+  if (temp > 0.0f)
+    n = block_normalise<T, kSampleThreads>(row, vocab, temp, top_k ? top_k[r] : -1, top_p ? top_p[r] : 1.0f,
+                                           scratch, select);
+  for (int v = threadIdx.x; v < vocab; v += kSampleThreads) out[v] = n.ok ? prob_at(row, v, temp, n) : 0.0f;
   if (threadIdx.x == 0) status[r] = n.ok ? RLT_ROW_OK : RLT_ROW_BAD_LOGITS;
 }
 
@@ -590,8 +778,8 @@ __device__ __forceinline__ int request_of_row(const int32_t* cu_rows, int n, int
   return lo;
 }
 
-template <typename T, int kThreads, bool kStaged>
-__global__ void __launch_bounds__(kThreads)
+template <typename T, int kThreads>
+__global__ void __launch_bounds__(kThreads, 3)
 row_stats_kernel(const T* __restrict__ target_logits, const T* __restrict__ draft_logits, int64_t row_stride,
                  int vocab, const int32_t* __restrict__ cu_rows, int n, const int32_t* __restrict__ row_counts,
                  const int64_t* __restrict__ tokens, int tokens_width, const float* __restrict__ temperature,
@@ -612,15 +800,8 @@ row_stats_kernel(const T* __restrict__ target_logits, const T* __restrict__ draf
   } else {
     if (side == 1 && j == count - 1) return;  // the bonus row has no draft distribution
     const T* logits = (side == 0 ? target_logits : draft_logits) + static_cast<int64_t>(row) * row_stride;
-    RowNorm norm;
-    if constexpr (kStaged) {
-      extern __shared__ __align__(16) float staged[];
-      norm = block_normalise<float, kThreads, true>(stage_row<T, kThreads>(logits, vocab, staged), vocab, temp,
-                                                    top_k ? top_k[i] : -1, top_p ? top_p[i] : 1.0f, scratch, select);
-    } else {
-      norm = block_normalise<T, kThreads>(logits, vocab, temp, top_k ? top_k[i] : -1, top_p ? top_p[i] : 1.0f,
-                                          scratch, select);
-    }
+    const RowNorm norm = block_normalise<T, kThreads>(logits, vocab, temp, top_k ? top_k[i] : -1, top_p ? top_p[i] : 1.0f, scratch,
+                                                      select);
     const int64_t d = j < count - 1 ? tokens[static_cast<int64_t>(i) * tokens_width + j + 1] : -1;
     out.m = norm.m;
     out.z = norm.z;
@@ -714,11 +895,6 @@ decide_kernel(const T* __restrict__ target_logits, const T* __restrict__ draft_l
   }
 }
 
-// Filters were passed and an fp32 copy of a row fits beside the kernels' static shared memory.
-bool stage_rows(const int32_t* top_k, const float* top_p, int vocab) {
-  return (top_k != nullptr || top_p != nullptr) && static_cast<size_t>(vocab) * sizeof(float) <= 200u * 1024u;
-}
-
 int check_logits(const void* logits, int64_t row_stride, int rows, int vocab, int dtype) {
   RLT_REQUIRE(dtype_valid(dtype), "acceptance: logits must be float32, float16 or bfloat16");
   RLT_REQUIRE(rows >= 0 && vocab > 0 && row_stride >= vocab, "acceptance: invalid logits shape");
@@ -774,19 +950,9 @@ extern "C" RLT_API int rlt_sample_rows(const void* logits, int64_t row_stride, i
   if (status != RLT_OK || rows == 0) return status;
   RLT_REQUIRE(temperature && uniforms && tokens && status_out, "sample_rows: null pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (stage_rows(top_k, top_p, vocab)) {
-    const size_t smem = static_cast<size_t>(vocab) * sizeof(float);
-    RLT_DISPATCH_DTYPE(dtype, T, {
-      auto kernel = sample_rows_kernel<T, true>;
-      RLT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      kernel<<<rows, kSampleThreads, smem, s>>>(static_cast<const T*>(logits), row_stride, vocab, temperature, top_k,
-                                                top_p, uniforms, tokens, status_out);
-    });
-  } else {
-    RLT_DISPATCH_DTYPE(dtype, T, (sample_rows_kernel<T, false><<<rows, kSampleThreads, 0, s>>>(
-                                     static_cast<const T*>(logits), row_stride, vocab, temperature, top_k, top_p,
-                                     uniforms, tokens, status_out)));
-  }
+  RLT_DISPATCH_DTYPE(dtype, T, (sample_rows_kernel<T><<<rows, kSampleThreads, 0, s>>>(
+                                   static_cast<const T*>(logits), row_stride, vocab, temperature, top_k, top_p,
+                                   uniforms, tokens, status_out)));
   return launch_status("sample_rows_kernel");
 }
 
@@ -798,19 +964,9 @@ extern "C" RLT_API int rlt_probabilities(const void* logits, int64_t row_stride,
   if (status != RLT_OK || rows == 0) return status;
   RLT_REQUIRE(temperature && probs && status_out, "probabilities: null pointer");
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  if (stage_rows(top_k, top_p, vocab)) {
-    const size_t smem = static_cast<size_t>(vocab) * sizeof(float);
-    RLT_DISPATCH_DTYPE(dtype, T, {
-      auto kernel = probabilities_kernel<T, true>;
-      RLT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      kernel<<<rows, kSampleThreads, smem, s>>>(static_cast<const T*>(logits), row_stride, vocab, temperature, top_k,
-                                                top_p, probs, status_out);
-    });
-  } else {
-    RLT_DISPATCH_DTYPE(dtype, T, (probabilities_kernel<T, false><<<rows, kSampleThreads, 0, s>>>(
-                                     static_cast<const T*>(logits), row_stride, vocab, temperature, top_k, top_p,
-                                     probs, status_out)));
-  }
+  RLT_DISPATCH_DTYPE(dtype, T, (probabilities_kernel<T><<<rows, kSampleThreads, 0, s>>>(
+                                   static_cast<const T*>(logits), row_stride, vocab, temperature, top_k, top_p,
+                                   probs, status_out)));
   return launch_status("probabilities_kernel");
 }
 
@@ -870,22 +1026,10 @@ extern "C" RLT_API int rlt_accept_rejection(const void* target_logits, const voi
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   RowStats* stats = static_cast<RowStats*>(workspace);
-  if (stage_rows(top_k, top_p, vocab)) {
-    const size_t smem = static_cast<size_t>(vocab) * sizeof(float);
-    RLT_DISPATCH_DTYPE(dtype, T, {
-      auto kernel = row_stats_kernel<T, kSampleThreads, true>;
-      RLT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-      kernel<<<dim3(rows, 2), kSampleThreads, smem, s>>>(static_cast<const T*>(target_logits),
-                                                         static_cast<const T*>(draft_logits), row_stride, vocab, cu_rows,
-                                                         n, row_counts, tokens, tokens_width, temperature, top_k, top_p,
-                                                         stats);
-    });
-  } else {
-    RLT_DISPATCH_DTYPE(dtype, T, (row_stats_kernel<T, kStatsThreads, false><<<dim3(rows, 2), kStatsThreads, 0, s>>>(
-                                     static_cast<const T*>(target_logits), static_cast<const T*>(draft_logits),
-                                     row_stride, vocab, cu_rows, n, row_counts, tokens, tokens_width, temperature,
-                                     top_k, top_p, stats)));
-  }
+  RLT_DISPATCH_DTYPE(dtype, T, (row_stats_kernel<T, kStatsThreads><<<dim3(rows, 2), kStatsThreads, 0, s>>>(
+                                   static_cast<const T*>(target_logits), static_cast<const T*>(draft_logits),
+                                   row_stride, vocab, cu_rows, n, row_counts, tokens, tokens_width, temperature,
+                                   top_k, top_p, stats)));
   status = launch_status("row_stats_kernel");
   if (status != RLT_OK) return status;
   RLT_DISPATCH_DTYPE(dtype, T, (decide_kernel<T><<<n, kSampleThreads, 0, s>>>(
