@@ -415,6 +415,18 @@ def test_expert_products(dtype, act, inner, outer, counts):
     close(got, want.cpu(), dtype, 2.0)
 
 
+@pytest.mark.parametrize("inner,outer", [(704, 520), (72, 136), (64, 2048)])
+@pytest.mark.parametrize("counts", [[700, 0, 257, 1, 1023], [33, 480, 225, 31], [2048] * 5])
+def test_expert_products_of_pairs_of_ctas(inner, outer, counts):
+    """Prompts: more tiles than pairs, row counts around the halves a pair takes, outputs that leave the second CTA of a pair with few or none."""
+    g = torch.Generator().manual_seed(outer)
+    x = torch.randn(sum(counts), inner, generator=g).bfloat16().cuda()
+    w = (torch.randn(len(counts), outer, inner, generator=g) / inner ** 0.5).bfloat16().cuda()
+    got = rlt.expert_gemm(x, w, torch.tensor(counts, dtype=torch.int32, device="cuda"))
+    want = torch.cat([rows.double() @ w[e].double().T for e, rows in enumerate(x.split(counts))])
+    close(got, want.cpu(), torch.bfloat16, 2.0)
+
+
 def test_the_mamba_scan_still_takes_its_own_decays():
     """Both forms of the recurrence share their kernels: driven by step sizes it is what it was."""
     g = torch.Generator().manual_seed(2)
