@@ -177,6 +177,29 @@ def test_block_epilogue(dtype, kv_heads, dim, vdim, ff, kind):
         close(out[:, 8:], plain.gelu(x) if kind == "gelu" else plain.gelu_tanh(x), dtype)
 
 
+@pytest.mark.parametrize("rows", [511, 512, 513, 515, 1030])
+@pytest.mark.parametrize("kv_heads,dim,ff", [(2, 64, 136), (3, 5, 17)])
+def test_block_epilogue_of_a_prompt(rows, kv_heads, dim, ff):
+    """Several rows per thread: a last thread with some of them, pages and padding rows among them."""
+    g = torch.Generator().manual_seed(rows)
+    width, pages = kv_heads * dim, -(-rows // BLOCK)
+    proj = torch.randn(rows, 2 * width + ff, generator=g).bfloat16().cuda()
+    order = torch.randperm(pages, generator=g).to(torch.int32)
+    row_seq = torch.zeros(rows, dtype=torch.int32)
+    row_seq[3::7] = -1
+    batch = SimpleNamespace(tables=order.cuda()[None, None], row_seq=row_seq.cuda(), positions=torch.arange(rows, dtype=torch.int32, device="cuda"))
+    key, value = (torch.full((pages, BLOCK, kv_heads, dim), 9.0, dtype=torch.bfloat16, device="cuda") for _ in range(2))
+    out = torch.full((rows + 1, ff), 9.0, dtype=torch.bfloat16, device="cuda")
+    rlt.block_epilogue(proj, batch, kv=(0, width, key, value), act=(2 * width, ff, "gelu", out[:rows], 0))
+    kept = row_seq.cuda() >= 0
+    for cache, column in ((key, 0), (value, width)):
+        rows_of = cache[order.long().cuda()].flatten(0, 1)
+        assert torch.equal(rows_of[:rows][kept], proj[:, column:column + width].view(rows, kv_heads, dim)[kept])
+        assert bool((rows_of[:rows][~kept] == 9.0).all()) and bool((rows_of[rows:] == 9.0).all())
+    close(out[:rows], plain.gelu(proj[:, 2 * width:].double().cpu()), torch.bfloat16)
+    assert bool((out[rows] == 9.0).all())
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 @pytest.mark.parametrize("kind", ["gelu", "gelu_tanh"])
 def test_activations_over_their_whole_range(dtype, kind):

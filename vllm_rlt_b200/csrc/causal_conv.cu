@@ -32,9 +32,11 @@ struct ConvArgs {
 };
 
 // A thread owns kVec neighbouring channels (or kActVec activation columns) for a tile of tokens.
+// Bound by memory as long as enough loads are in flight: 16384 rows of 6144 channels (403 MB) take 104 us, 4352 channels beside 8448 gelu
+// columns (839 MB) 201 us; with a bound checked per token, spilled registers and two rows of activations ahead, 116 and 236 us.
 // kTaps 0: any number of taps, inputs re-read (from L1) for every output, one channel per thread.
 template <typename T, int kTaps, int kVec, int kActVec>
-__global__ void __launch_bounds__(kThreads, 8)
+__global__ void __launch_bounds__(kThreads, 6)
 causal_conv_kernel(ConvArgs a) {
   const int seq = blockIdx.z, first = blockIdx.y * kTile;
   const int row0 = a.cu[seq], n = a.cu[seq + 1] - row0;
@@ -45,13 +47,22 @@ causal_conv_kernel(ConvArgs a) {
     if (c >= a.act_width) return;
     const T* src = static_cast<const T*>(a.act_in) + (row0 + first) * a.in_stride + c;
     T* dst = static_cast<T*>(a.act_out) + (row0 + first) * a.act_out_stride + c;
-#pragma unroll 2
-    for (int i = 0; i < count; ++i) {
-      float v[kActVec];
-      load_floats<T, kActVec>(src + i * a.in_stride, v);
+    struct alignas(sizeof(T) * kActVec) ActVec { T e[kActVec]; };
+    constexpr int kAhead = 4;               // rows in flight per thread
+    for (int base = 0; base < count; base += kAhead) {
+      ActVec next[kAhead];
 #pragma unroll
-      for (int e = 0; e < kActVec; ++e) v[e] = activate<T>(v[e], a.act);
-      store_floats<T, kActVec>(dst + i * a.act_out_stride, v);
+      for (int i = 0; i < kAhead; ++i)
+        if (base + i < count) next[i] = *reinterpret_cast<const ActVec*>(src + (base + i) * a.in_stride);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i)
+        if (base + i < count) {
+          float v[kActVec];
+#pragma unroll
+          for (int e = 0; e < kActVec; ++e) v[e] = Elem<T>::to_float(next[i].e[e]);
+          activate_all<T, kActVec>(v, a.act);
+          store_floats<T, kActVec>(dst + (base + i) * a.act_out_stride, v);
+        }
     }
     return;
   }
@@ -87,30 +98,40 @@ causal_conv_kernel(ConvArgs a) {
 #pragma unroll
       for (int e = 0; e < kVec; ++e) window[j + 1][e] = Elem<T>::to_float(x.e[e]);
     }
-    constexpr int kAhead = 4;
-    Vec next[kAhead];
-    for (int base = 0; base < count; base += kAhead) {
+    const T* src = in + first * a.in_stride;
+    T* dst = out + first * a.out_stride;
+    auto output = [&](const Vec& x, int i) {
+      float sum[kVec];
 #pragma unroll
-      for (int i = 0; i < kAhead; ++i)
-        if (base + i < count) next[i] = *reinterpret_cast<const Vec*>(in + (first + base + i) * a.in_stride);
+      for (int e = 0; e < kVec; ++e) {
 #pragma unroll
-      for (int i = 0; i < kAhead; ++i) {
-        if (base + i < count) {
-          float sum[kVec];
+        for (int j = 0; j + 1 < kTaps; ++j) window[j][e] = window[j + 1][e];
+        window[kTaps - 1][e] = Elem<T>::to_float(x.e[e]);
+        sum[e] = 0.0f;
 #pragma unroll
-          for (int e = 0; e < kVec; ++e) {
-#pragma unroll
-            for (int j = 0; j + 1 < kTaps; ++j) window[j][e] = window[j + 1][e];
-            window[kTaps - 1][e] = Elem<T>::to_float(next[i].e[e]);
-            sum[e] = 0.0f;
-#pragma unroll
-            for (int j = 0; j < kTaps; ++j) sum[e] = fmaf(wr[e][j], window[j][e], sum[e]);
-            sum[e] = silu(sum[e] + bias[e]);
-          }
-          store_floats<T, kVec>(out + (first + base + i) * a.out_stride, sum);
-        }
+        for (int j = 0; j < kTaps; ++j) sum[e] = fmaf(wr[e][j], window[j][e], sum[e]);
+        sum[e] = silu(sum[e] + bias[e]);
       }
+      store_floats<T, kVec>(dst + i * a.out_stride, sum);
+    };
+    // Groups of kAhead tokens without a bound to check, the next group's inputs on their way while one is computed.
+    constexpr int kAhead = 4;
+    const int groups = count / kAhead;
+    Vec now[kAhead], next[kAhead];
+    auto load = [&](Vec (&to)[kAhead], int group) {
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) to[i] = *reinterpret_cast<const Vec*>(src + (group * kAhead + i) * a.in_stride);
+    };
+    if (groups > 0) load(now, 0);
+#pragma unroll 1
+    for (int g = 0; g < groups; ++g) {
+      if (g + 1 < groups) load(next, g + 1);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) output(now[i], g * kAhead + i);
+#pragma unroll
+      for (int i = 0; i < kAhead; ++i) now[i] = next[i];
     }
+    for (int i = groups * kAhead; i < count; ++i) output(*reinterpret_cast<const Vec*>(src + i * a.in_stride), i);
   } else {
     static_assert(kTaps > 0 || kVec == 1, "the re-reading form handles one channel per thread");
     for (int i = 0; i < count; ++i) {
@@ -139,8 +160,7 @@ conv_step_kernel(ConvArgs a) {
     if (c >= a.act_width) return;
     float v[kVec];
     load_floats<T, kVec>(static_cast<const T*>(a.act_in) + row * a.in_stride + c, v);
-#pragma unroll
-    for (int e = 0; e < kVec; ++e) v[e] = activate<T>(v[e], a.act);
+    activate_all<T, kVec>(v, a.act);
     store_floats<T, kVec>(static_cast<T*>(a.act_out) + row * a.act_out_stride + c, v);
     return;
   }

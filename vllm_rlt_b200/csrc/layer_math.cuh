@@ -52,6 +52,38 @@ __device__ __forceinline__ float activate(float x, int act) {
   return 0.5f * x * (1.0f + tanhf(u));
 }
 
+// gelu with erf_approx for two values of a 16-bit result, two at a time in the packed unit: 20 instructions instead of 40, which is what bounds
+// streaming activations (16384 rows of 8448 columns need 84 us of issue slots one by one, 86 us of memory traffic).
+__device__ __forceinline__ float2 gelu_erf_pair(float2 x) {
+  const float2 u = mul_pair(x, make_float2(0.70710678118654752f, 0.70710678118654752f)), z = make_float2(fabsf(u.x), fabsf(u.y)), one = make_float2(1.0f, 1.0f);
+  const float2 d = fma_pair(make_float2(0.3275911f, 0.3275911f), z, one);
+  const float2 t = make_float2(__fdividef(1.0f, d.x), __fdividef(1.0f, d.y));
+  float2 p = fma_pair(t, make_float2(1.061405429f, 1.061405429f), make_float2(-1.453152027f, -1.453152027f));
+  p = fma_pair(t, p, make_float2(1.421413741f, 1.421413741f));
+  p = fma_pair(t, p, make_float2(-0.284496736f, -0.284496736f));
+  p = mul_pair(t, fma_pair(t, p, make_float2(0.254829592f, 0.254829592f)));
+  const float2 w = mul_pair(mul_pair(z, z), make_float2(-1.4426950408889634f, -1.4426950408889634f));
+  const float2 q = fma_pair(mul_pair(p, make_float2(-1.0f, -1.0f)), make_float2(fast_exp2(w.x), fast_exp2(w.y)), one);
+  const float2 half = mul_pair(x, make_float2(0.5f, 0.5f));
+  return fma_pair(half, make_float2(copysignf(q.x, u.x), copysignf(q.y, u.y)), half);
+}
+template <typename T, int kVec>
+__device__ __forceinline__ void activate_all(float (&v)[kVec], int act) {
+  if constexpr (sizeof(T) == 2 && kVec % 2 == 0) {
+    if (act == kActGeluErf) {
+#pragma unroll
+      for (int e = 0; e < kVec; e += 2) {
+        const float2 y = gelu_erf_pair(make_float2(v[e], v[e + 1]));
+        v[e] = y.x;
+        v[e + 1] = y.y;
+      }
+      return;
+    }
+  }
+#pragma unroll
+  for (int e = 0; e < kVec; ++e) v[e] = activate<T>(v[e], act);
+}
+
 // kVec consecutive elements as fp32, in one access of kVec * sizeof(T) bytes (the caller guarantees the alignment).
 template <typename T, int kVec>
 __device__ __forceinline__ void load_floats(const T* p, float (&v)[kVec]) {
