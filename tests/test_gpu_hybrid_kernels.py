@@ -327,6 +327,28 @@ def test_long_prompts_run_in_segments(p, size):
     assert torch.equal(state[2], start[2])
 
 
+@pytest.mark.parametrize("heads,p,size,groups", [(4, 64, 128, 2), (3, 40, 72, 3), (2, 136, 96, 1)])
+def test_scan_of_whole_and_partial_chunks(heads, p, size, groups):
+    """Whole chunks come as boxes, a sequence's last piece row by row, with zeros behind it and behind a head's columns."""
+    lengths = [256, 128, 127, 129, 20, 384]
+    inputs = scan_inputs(sum(lengths), heads, p, size, groups, torch.bfloat16, 6)
+    x, b, c, dt, dt_bias, a_log, d = inputs
+    state = torch.randn(len(lengths), heads, size, p, device="cuda")
+    start = state.clone()
+    wide = torch.cat([x, b, c], 1).cuda()
+    out = torch.empty(sum(lengths), heads * p, dtype=torch.bfloat16, device="cuda")
+    xs, bs, cs = wide.split((heads * p, groups * size, groups * size), 1)
+    rlt.ssd_scan(xs, bs, cs, dt.cuda(), dt_bias.cuda(), a_log.cuda(), d.cuda(), state, out, group_of(lengths, [9] * len(lengths), range(len(lengths))))
+    at = 0
+    for s, n in enumerate(lengths):
+        part = [t[at:at + n].double() for t in (x, b, c, dt)]
+        y, final = plain.recurrence(part[0].view(n, heads, p), part[1].view(n, groups, size), part[2].view(n, groups, size), part[3],
+                                    dt_bias.double(), a_log.double(), d.double(), start[s].double().cpu())
+        close(out[at:at + n], y.reshape(n, -1), torch.bfloat16)
+        close(state[s], final, torch.float32, 20.0)
+        at += n
+
+
 def test_kernels_refuse_what_they_cannot_do():
     with pytest.raises(ValueError, match="multiple"):
         rlt.B200PagedAttention().scored(torch.zeros(1, 3, 16, device="cuda"), torch.zeros(1, 3, 16, device="cuda"),

@@ -11,6 +11,10 @@
 // y = 2^L (C S) + M X + d x is stored from registers; the state S = 2^L_end S + D lives in fp32 registers (32 per thread)
 // for the whole sequence.  W takes the room of C once the products of C are complete.  113 KiB of shared memory and 256
 // TMEM columns: two CTAs per SM, each covering the other's copies and waits.
+//
+// What bounds it is the chain of a chunk's phases.  So operands of whole chunks come as boxes, which keep no thread busy; step sizes are
+// loaded a chunk ahead (a third of a chunk went into waiting for them); and rows of y leave in pieces of 64 bytes.  16384 tokens of 64 heads
+// of 64 x 128 in 8 sequences: 324 -> 248 us; 8191 tokens of 16 heads of 128 x 128 with constant decays: 121 -> 113 us.
 #include "sm100_primitives.cuh"
 #include "ssd_scan.cuh"
 
@@ -30,7 +34,7 @@ struct ScanShared {
   unsigned char x[kRows * 128];         // [token][64]
   unsigned char s_hi[kRows * 128], s_lo[kRows * 128];   // [state row][64]
   float log_weight[kRows];              // L - log2(dt): M = G 2^(L_q - this), W = X 2^(L_end - this)
-  unsigned long long g_done, y_done, mx_done, d_done;
+  unsigned long long loaded, g_done, y_done, mx_done, d_done;
   uint32_t tmem_base;
 };
 
@@ -46,7 +50,7 @@ __device__ __forceinline__ void split_pair(float a, float b, uint32_t* hi, uint3
 
 template <bool kOutput>
 __global__ void __launch_bounds__(kThreads, 2)
-scan_umma_kernel(ScanArgs a) {
+scan_umma_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap b_map, const __grid_constant__ CUtensorMap c_map, ScanArgs a) {
   extern __shared__ __align__(1024) unsigned char smem_raw[];
   ScanShared& sm = *reinterpret_cast<ScanShared*>(smem_raw);
   const int lane = threadIdx.x & 31, warp = __shfl_sync(0xffffffffu, static_cast<int>(threadIdx.x >> 5), 0);
@@ -74,6 +78,7 @@ scan_umma_kernel(ScanArgs a) {
   auto segment_decay = [&](int s) { return a.segment_decay + (static_cast<int64_t>(seq) * kMaxSegments + s) * a.heads + head; };
 
   if (threadIdx.x == 0) {
+    mbar_init(smem_u32(&sm.loaded), 1);
     mbar_init(smem_u32(&sm.g_done), 1);
     mbar_init(smem_u32(&sm.y_done), 1);
     mbar_init(smem_u32(&sm.mx_done), 1);
@@ -133,7 +138,7 @@ scan_umma_kernel(ScanArgs a) {
   const T* xg = static_cast<const T*>(a.x) + static_cast<int64_t>(head) * a.p + p0;
   const T* bg = static_cast<const T*>(a.b) + static_cast<int64_t>(group) * a.n;
   const T* cg = static_cast<const T*>(a.c) + static_cast<int64_t>(group) * a.n;
-  const T* dtg = static_cast<const T*>(a.dt) + head;
+  const uint16_t* dtg = static_cast<const uint16_t*>(a.dt) + head;
   const int p_valid = min(kCols, a.p - p0);
   auto load_wide = [&](unsigned char (&dst)[2][kRows * 128], const T* src, int count) {   // state columns in two halves of 64
     for (int i = threadIdx.x; i < kRows * 16; i += kThreads) {
@@ -149,18 +154,42 @@ scan_umma_kernel(ScanArgs a) {
   float segment_log = 0.0f;
   bool failed = false;
   uint32_t tmem = 0;
+  uint32_t dt_raw[4] = {0u, 0u, 0u, 0u};             // the coming chunk's step sizes, four tokens per lane (a word each: pairs would be joined on arrival)
+  auto load_dt = [&](int from) {
+    if (constant) return;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (from + 4 * lane + i < last) dt_raw[i] = dtg[(static_cast<int64_t>(row0) + from + 4 * lane + i) * a.dt_stride];
+  };
+  load_dt(first);
 
   for (int base = first, chunk = 0; base < last; base += kRows, ++chunk) {
     const int count = min(kRows, last - base);
     const int64_t first_row = row0 + base;
     const uint32_t parity = chunk & 1;
     bool ok = true;
-    load_wide(sm.b, bg + first_row * a.xbc_stride, count);
-    if (kOutput) load_wide(sm.c, cg + first_row * a.xbc_stride, count);
-    for (int i = threadIdx.x; i < kRows * 8; i += kThreads) {
-      const int r = i >> 3, q = i & 7;
-      const bool live = r < count && q * 8 < p_valid;
-      copy_piece(smem_u32(sm.x + swizzled(r, q)), live ? xg + (first_row + r) * a.xbc_stride + q * 8 : xg, live);
+    const bool whole = count == kRows;               // every chunk but a sequence's last: boxes; rows behind the last token have to read as zero
+    if (whole) {
+      if (threadIdx.x == 0) {
+        const uint32_t bar = smem_u32(&sm.loaded);
+        const int at = static_cast<int>(first_row);
+        fence_async_proxy();
+        mbar_expect_tx(bar, (kOutput ? 5 : 3) * kRows * 128);
+#pragma unroll
+        for (int h = 0; h < 2; ++h) tma_load_3d(smem_u32(sm.b[h]), &b_map, h * 64, group, at, bar);
+        if (kOutput)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) tma_load_3d(smem_u32(sm.c[h]), &c_map, h * 64, group, at, bar);
+        tma_load_3d(smem_u32(sm.x), &x_map, p0, head, at, bar);
+      }
+    } else {
+      load_wide(sm.b, bg + first_row * a.xbc_stride, count);
+      if (kOutput) load_wide(sm.c, cg + first_row * a.xbc_stride, count);
+      for (int i = threadIdx.x; i < kRows * 8; i += kThreads) {
+        const int r = i >> 3, q = i & 7;
+        const bool live = r < count && q * 8 < p_valid;
+        copy_piece(smem_u32(sm.x + swizzled(r, q)), live ? xg + (first_row + r) * a.xbc_stride + q * 8 : xg, live);
+      }
     }
     // L of all 128 tokens, four per lane; every warp computes it, so nobody waits for another warp's
     float log_row, log_end;
@@ -170,10 +199,11 @@ scan_umma_kernel(ScanArgs a) {
       for (int i = 0; i < 4; ++i) {
         const int token = 4 * lane + i;
         if (constant) dt[i] = token < count ? 1.0f : 0.0f;
-        else dt[i] = token < count ? softplus(Elem<T>::to_float(dtg[(first_row + token) * a.dt_stride]) + dt_bias) : 0.0f;
+        else dt[i] = token < count ? softplus(__uint_as_float(dt_raw[i] << 16) + dt_bias) : 0.0f;
         sum += rate * dt[i];
         l[i] = sum;
       }
+      load_dt(base + kRows);
       float before = sum;
 #pragma unroll
       for (int x = 1; x < 32; x <<= 1) {
@@ -197,6 +227,10 @@ scan_umma_kernel(ScanArgs a) {
     tcgen05_before_sync();
     __syncthreads();
     tcgen05_after_sync();
+    if (whole) {
+      ok = mbar_wait(smem_u32(&sm.loaded), parity);
+      __syncwarp();
+    }
     if (chunk == 0) tmem = sm.tmem_base;
     const uint32_t tmem_row = tmem + (static_cast<uint32_t>(wr * 32) << 16);
 
@@ -305,15 +339,24 @@ scan_umma_kernel(ScanArgs a) {
       tmem_load32(tmem_row + kColY + col0, in);
       tmem_load_wait();
       const float scale = fast_exp2(log_row);
-      T* yg = static_cast<T*>(a.y) + (first_row + row) * a.y_stride + static_cast<int64_t>(head) * a.p + p0 + col0;
+      // through the warp's own part of s_hi (C S is done, the new state comes later), so that four lanes store 64 bytes of a row
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         float v[8];
         load_floats<T, 8>(reinterpret_cast<const T*>(sm.x + swizzled(row, half * 4 + q)), v);
 #pragma unroll
         for (int e = 0; e < 8; ++e) v[e] = fmaf(skip, v[e], fmaf(scale, cs[q * 8 + e], __uint_as_float(in[q * 8 + e])));
-        if (row < count && col0 + q * 8 < p_valid) store_floats<T, 8>(yg + q * 8, v);
+        store_floats<T, 8>(reinterpret_cast<T*>(sm.s_hi + swizzled(row, half * 4 + q)), v);
       }
+      __syncwarp();
+      const int piece = lane & 3, column = col0 + piece * 8;
+      T* yg = static_cast<T*>(a.y) + first_row * a.y_stride + static_cast<int64_t>(head) * a.p + p0 + column;
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const int r = wr * 32 + i * 8 + (lane >> 2);
+        if (r < count && column < p_valid) *reinterpret_cast<uint4*>(yg + r * a.y_stride) = *reinterpret_cast<const uint4*>(sm.s_hi + swizzled(r, half * 4 + piece));
+      }
+      __syncwarp();
     }
     ok = mbar_wait(smem_u32(&sm.d_done), parity) && ok;
     __syncwarp();
@@ -352,11 +395,11 @@ scan_umma_kernel(ScanArgs a) {
 }
 
 template <bool kOutput>
-int launch_one(const ScanArgs& a, int sequences, cudaStream_t stream) {
+int launch_one(const ScanArgs& a, const CUtensorMap (&maps)[3], int sequences, cudaStream_t stream) {
   auto kernel = scan_umma_kernel<kOutput>;
   RLT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(sizeof(ScanShared))));
   const dim3 grid(static_cast<unsigned>(a.heads), static_cast<unsigned>(sequences * ((a.p + kCols - 1) / kCols)), static_cast<unsigned>(a.segment_count));
-  kernel<<<grid, kThreads, sizeof(ScanShared), stream>>>(a);
+  kernel<<<grid, kThreads, sizeof(ScanShared), stream>>>(maps[0], maps[1], maps[2], a);
   return launch_status("scan_umma_kernel");
 }
 
@@ -369,12 +412,20 @@ bool scan_umma_supported(const ScanArgs& a) {
 }
 
 int launch_scan_umma(const ScanArgs& a, int sequences, cudaStream_t stream) {
+  // [rows, heads or groups, columns]: a box leaves what lies behind a head's columns zero.  Only whole chunks of a sequence's own rows are read
+  // through the maps, so the number of rows, which only the device knows, is left open.
+  const int64_t rows = 0x7fffffff;
+  CUtensorMap maps[3];
+  if (make_box_map<3>(&maps[0], a.x, {a.p, a.heads, rows}, {1, a.p, a.xbc_stride}, {64, 1, kRows}) != RLT_OK ||
+      make_box_map<3>(&maps[1], a.b, {a.n, a.groups, rows}, {1, a.n, a.xbc_stride}, {64, 1, kRows}) != RLT_OK ||
+      make_box_map<3>(&maps[2], a.c, {a.n, a.groups, rows}, {1, a.n, a.xbc_stride}, {64, 1, kRows}) != RLT_OK)
+    return RLT_ERR_UNSUPPORTED;
   RLT_CUDA_TRY(cudaMemsetAsync(a.error, 0, sizeof(unsigned), stream));
   if (a.segment_count > 1) {
-    const int status = launch_one<false>(a, sequences, stream);
+    const int status = launch_one<false>(a, maps, sequences, stream);
     if (status != RLT_OK) return status;
   }
-  return launch_one<true>(a, sequences, stream);
+  return launch_one<true>(a, maps, sequences, stream);
 }
 
 }  // namespace rlt

@@ -199,7 +199,10 @@ int run_scan(ScanArgs& a, int sequences, int max_tokens, int dtype, void* worksp
     a.segments = reinterpret_cast<float*>(static_cast<unsigned char*>(workspace) + 256);
     a.segment_decay = a.segments + static_cast<size_t>(sequences) * (kMaxSegments + 1) * a.heads * a.n * a.p;
   }
-  if (scan_umma_supported(a)) return launch_scan_umma(a, sequences, s);
+  if (scan_umma_supported(a)) {
+    const int launched = launch_scan_umma(a, sequences, s);
+    if (launched != RLT_ERR_UNSUPPORTED) return launched;
+  }
   return launch_scan_chunks(a, sequences, s);
 }
 
