@@ -306,6 +306,24 @@ def test_delta_rule_of_unequal_portions(dtype):
     assert torch.equal(state[2].cpu(), before[2]) and torch.equal(state[4].cpu(), before[4])
 
 
+@pytest.mark.parametrize("offset,pad", [(0, 8), (1, 0), (0, 3), (8, 8)])
+def test_delta_rule_takes_decays_of_any_alignment(offset, pad):
+    """Rows of decays that no 16-byte piece fits are read element by element, to the same bits."""
+    heads, dim, n = 2, 64, 150
+    case, a_log, dt_bias = delta_case(n, heads, heads, dim, dim, torch.bfloat16, 4)
+    q, k, v, decay, beta = (t.cuda() for t in case[:5])
+    qkv, width = torch.cat([q, k, v], 1), heads * dim
+    wide = torch.full((n * (width + pad) + offset,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    shifted = wide[offset:].view(n, width + pad)[:, :width]
+    shifted.copy_(decay)
+    outs = []
+    for raw in (decay, shifted):
+        state, out = torch.zeros(1, heads, dim, dim, device="cuda"), torch.empty(n, width, dtype=torch.bfloat16, device="cuda")
+        rlt.delta_scan(*qkv.split(width, 1), raw, beta, dt_bias.cuda(), a_log.cuda(), state, out, group_of([n], [0], [0]))
+        outs.append((state, out))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+
+
 # ---- experts ----------------------------------------------------------------------------------------
 @pytest.mark.parametrize("rows,experts,top", [(1, 4, 1), (17, 16, 4), (300, 60, 6), (5000, 9, 9), (40, 200, 3)])
 def test_routing_by_biased_logits(rows, experts, top):

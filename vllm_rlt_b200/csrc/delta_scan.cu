@@ -232,6 +232,7 @@ extern "C" RLT_API int rlt_delta_scan(const void* q, const void* k, const void* 
     a.error = static_cast<unsigned*>(workspace);         // workspace: an error word (256 bytes), then the records
     a.records = static_cast<unsigned char*>(workspace) + 256;
     int64_t records;
+    a.decay_pieces = decay_stride % 8 == 0 && aligned16(decay);   // dim % 8 == 0 here
     a.chunk_count = pass_chunks(sequences, max_tokens, rows, heads, dim, &records);
     RLT_CUDA_TRY(cudaMemsetAsync(a.error, 0, sizeof(unsigned), s));
     for (a.first_chunk = 0; a.first_chunk * kChunk < max_tokens; a.first_chunk += a.chunk_count) {

@@ -10,6 +10,7 @@ constexpr float kUnitEps = 1e-6f;      // inside the root of a unit vector's len
 struct DeltaArgs {
   const void* q; const void* k; const void* v; int64_t qkv_stride;    // [rows, stride]: q, k [kv_heads * dim], v [heads * vdim]
   const void* decay; int64_t decay_stride;                            // raw decays [rows, heads * dim]
+  bool decay_pieces;                                                  // chunk kernels: 16 bytes of them at a time (aligned rows)
   const void* beta; int64_t beta_stride;                              // raw write strengths [rows, heads]
   const float* dt_bias; const float* a_log;                           // [heads * dim], [heads]
   void* out; int64_t out_stride;                                      // [rows, heads * vdim]
