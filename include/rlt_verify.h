@@ -749,6 +749,15 @@ RLT_API int rlt_delta_scan(const void* q, const void* k, const void* v, int64_t 
                    int max_tokens, int rows, int heads, int kv_heads, int dim, int vdim, int dtype, void* workspace, size_t workspace_bytes,
                    rlt_stream_t stream);
 
+/* Host only: the metadata of an engine step into `words`, in the order sequence by sequence.  at: offsets into `words` of tokens (int64 [rows]),
+ * positions, row_seq and previous (int32 [rows]: position of each row's token, its sequence, the token before it), cu [sequences + 1], the same from
+ * sequence `short_sequences` on counted from there, starts, lengths, slots [sequences], and page tables [planes][sequences][width].  records
+ * [portions][5 + 2 planes]: address of the portion's int64 tokens, their number, tokens stored before, slot, the last of them (-1: none), then per
+ * plane the address of the int32 page ids and their number (those beyond width are left out, the rest of a table row is zero).  Sequences behind
+ * the portions are padding: one row, row_seq -1, previous -1, length 0, dummy_slot.  RLT_ERR_INVALID where `rows` is not what they add up to. */
+RLT_API int rlt_step_metadata(int32_t* words, const int64_t* at, const int64_t* records, int portions, int sequences, int planes, int width,
+                      int short_sequences, int64_t rows, int64_t dummy_slot);
+
 #ifdef __cplusplus
 }
 #endif

@@ -188,6 +188,46 @@ def test_steps_mix_portions_and_single_tokens(counting_engine):
     assert engine.step([dict(name="a", tokens=a[42:43])]).shape == (0, 53)
 
 
+@pytest.mark.parametrize("counts, starts, padding", [([1], [0], 0), ([1, 1, 1], [0, 7, 40], 5), ([16, 1, 17], [3, 0, 0], 0), ([2, 33, 40], [5, 0, 16], 0), ([], [], 4)])
+def test_step_metadata_is_what_a_loop_over_the_tokens_says(counts, starts, padding):
+    engine = rlt.Engine(CountingModel(), cuda_graphs=False, max_tokens=256, max_sequences=3)
+    cache, entries, rows, cu, previous = engine.cache, [], [], [0], []
+    for i, (n, start) in enumerate(zip(counts, starts)):
+        tokens, last = prompt(i, n, 53), 50 + i if start else -1
+        cache.admit(i)
+        cache.reserve(i, start + n)
+        if start:
+            cache.advance(i, start, last)
+        entries.append(rlt.StepEntry(i, tokens))
+        rows += [(t, start + at, i) for at, t in enumerate(tokens)]
+        previous += [last, *tokens[:-1]]
+        cu.append(len(rows))
+    rows += [(0, 0, -1)] * padding
+    previous += [-1] * padding
+    cu += range(cu[-1] + 1, cu[-1] + padding + 1)
+    short = sum(n <= engine_module.SHORT_PORTION for n in counts) + padding
+    layout = engine_module._Layout(len(rows), len(counts) + padding, 1, 4, short)
+    buffer = torch.zeros(layout.size, dtype=torch.int32)
+    engine._fill(layout, buffer, entries)
+    v = layout.views(buffer)
+    assert [v[k].tolist() for k in ("tokens", "positions", "row_seq")] == [list(c) for c in zip(*rows)]
+    assert v["previous"].tolist() == previous and v["cu"].tolist() == cu and v["long_cu"].tolist() == [c - cu[short] for c in cu[short:]]
+    assert v["starts"].tolist() == starts + [0] * padding and v["lengths"].tolist() == [a + n for a, n in zip(starts, counts)] + [0] * padding
+    assert v["slots"].tolist() == [cache.slot(i) for i in range(len(counts))] + [cache.dummy_slot] * padding
+    assert v["tables"][0].tolist() == [(cache.pages(i) + [0] * 4)[:4] for i in range(len(counts))] + [[0] * 4] * padding
+
+
+def test_tokens_of_other_kinds_are_taken_as_whole_numbers(counting_engine):
+    engine, tokens = counting_engine(), prompt(3, 20, 53)
+    for name, other in enumerate((tuple(tokens), [float(t) for t in tokens], [torch.tensor(t) for t in tokens])):
+        assert engine.step([dict(name=name, tokens=other, want=[19])]).argmax(-1).tolist() == expected_output(tokens, 1)
+        engine.release(name)
+    for bad in (53, -1, 2 ** 70, float("nan")):
+        for length in (1, 16, 30):
+            with pytest.raises(ValueError, match="vocabulary"):
+                engine.step([dict(name="a", tokens=[1] * (length - 1) + [bad])])
+
+
 def test_a_step_that_does_not_fit_changes_nothing(counting_engine):
     engine = counting_engine(max_tokens=64, max_sequences=2)
     engine.step([dict(name="a", tokens=[1] * 40)])

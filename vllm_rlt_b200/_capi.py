@@ -93,6 +93,7 @@ SIGNATURES = {
     "rlt_delta_scan_workspace_bytes": (_Z, [_I, _I, _I, _I, _I, _I, _I]),
     "rlt_delta_scan": (_I, [_P, _P, _P, _L, _P, _L, _P, _L, _P, _P, _P, _L, _P, _L, _P, _P, _P, _I, _I, _I, _I, _I, _I, _I, _I, _P, _Z, _P]),
     "rlt_rollback": (_I, [_P, _P, _I, _P, _I, _I, _I, _P, _P, _L, _P, _I, _P, _P, _P, _P, _P, _P]),
+    "rlt_step_metadata": (_I, [_P, _P, _P, _I, _I, _I, _I, _I, _L, _L]),
 }
 
 _lib = None

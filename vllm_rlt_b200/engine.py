@@ -9,11 +9,13 @@ and draw.  Steps in which every sequence decodes one token are replayed from a C
 
 from __future__ import annotations
 
+from array import array
 from collections import deque
 from dataclasses import dataclass, field
 
 import torch
 
+from . import _capi
 from .runner import Request, SamplingParams
 from .sequence_cache import CacheFull, SequenceCache
 from .speculative import argmax_rows, raise_for_status, round_uniforms, sample_rows
@@ -28,6 +30,28 @@ class StepEntry:
     name: object
     tokens: list
     want: list = field(default_factory=list)
+
+
+class _Portion:
+    """An entry whose tokens have been looked at: the tokens as 64-bit words."""
+
+    __slots__ = ("name", "tokens")
+
+    def __init__(self, entry: StepEntry, vocab: int):
+        self.name, tokens = entry.name, entry.tokens
+        try:
+            self.tokens = array("q", tokens if type(tokens) in (list, tuple) else list(tokens))
+        except (TypeError, OverflowError):                 # numbers of other kinds, or beyond any vocabulary
+            self.tokens = array("q", [int(t) if 0 <= t < vocab else -1 for t in tokens])
+        if len(self.tokens) == 1:
+            inside = 0 <= self.tokens[0] < vocab
+        elif len(self.tokens) <= SHORT_PORTION:
+            inside = all(0 <= t < vocab for t in self.tokens)
+        else:
+            low, high = torch.frombuffer(self.tokens, dtype=torch.int64).aminmax()
+            inside = low >= 0 and high < vocab
+        if not inside:
+            raise ValueError(f"entry {entry.name!r}: token outside the vocabulary")
 
 
 @dataclass
@@ -180,29 +204,26 @@ class Engine:
         their `want`.  A sequence is admitted at its first entry.  On `CacheFull` or a bad entry nothing has run."""
         entries = [e if isinstance(e, StepEntry) else StepEntry(**e) for e in entries]
         vocab = self.model.vocab_size
-        names = set()
+        portions = {}
         for e in entries:
-            if not e.tokens or e.name in names:
+            if not e.tokens or e.name in portions:
                 raise ValueError(f"entry {e.name!r}: every entry needs tokens and a sequence of its own")
-            names.add(e.name)
-            if not all(0 <= t < vocab for t in e.tokens):
-                raise ValueError(f"entry {e.name!r}: token outside the vocabulary")
+            portions[e.name] = _Portion(e, vocab)
             if not all(0 <= w < len(e.tokens) for w in e.want):
                 raise ValueError(f"entry {e.name!r}: wanted place outside the portion")
         if not entries:
             return torch.empty(0, vocab, device=self.device)
-        self._claim(entries)
-        order = sorted(range(len(entries)), key=lambda i: len(entries[i].tokens) > SHORT_PORTION)
-        ordered = [entries[i] for i in order]
+        self._claim(portions.values())
+        ordered = sorted(portions.values(), key=lambda p: len(p.tokens) > SHORT_PORTION)
         decode = self.cuda_graphs and all(len(e.tokens) == 1 for e in ordered)
         logits = self._decode_step(ordered) if decode else self._eager_step(ordered, entries)
-        for e in entries:
-            self.cache.advance(e.name, len(e.tokens), e.tokens[-1])
+        for p in ordered:
+            self.cache.advance(p.name, len(p.tokens), p.tokens[-1])
         self.steps += 1
         if decode:
             picked = [i for i, e in enumerate(entries) for _ in e.want]
             if picked != list(range(len(entries))):
-                logits = logits[torch.tensor(picked, dtype=torch.int64, device=self.device)]
+                logits = logits[self._indices(picked)]
         return logits
 
     def _claim(self, entries):
@@ -211,49 +232,46 @@ class Engine:
         fresh = [e.name for e in entries if e.name not in cache]
         if len(fresh) > cache.free_slots:
             raise CacheFull(f"{len(fresh)} new sequences, {cache.free_slots} free slots")
-        need = 0
+        need, growing = 0, []
         for e in entries:
-            held, length = (len(cache.pages(e.name)), cache.length(e.name)) if e.name in cache else (0, 0)
-            if length + len(e.tokens) > self.max_sequence_tokens:
+            length, held = cache.extent(e.name)
+            length += len(e.tokens)
+            if length > self.max_sequence_tokens:
                 raise CacheFull(f"sequence {e.name!r} would exceed {self.max_sequence_tokens} tokens")
-            need += max(cache.pages_for(length + len(e.tokens)) - held * cache.spec.planes, 0)
+            more = cache.pages_for(length) - held * cache.spec.planes
+            if more > 0:
+                need += more
+                growing.append((e.name, length))
         if need > cache.free_pages:
             raise CacheFull(f"{need} pages asked, {cache.free_pages} free")
-        for e in entries:
-            if e.name not in cache:
-                cache.admit(e.name)
-            cache.reserve(e.name, cache.length(e.name) + len(e.tokens))
+        for name in fresh:
+            cache.admit(name)
+        for name, length in growing:
+            cache.reserve(name, length)
 
-    def _fill(self, layout: _Layout, host: torch.Tensor, entries) -> None:
-        cache, v = self.cache, layout.views(host)
-        rows, tokens, positions, row_seq, previous, cu, starts, lengths, slots = 0, [], [], [], [], [0], [], [], []
-        for i, e in enumerate(entries):
-            n, start = len(e.tokens), cache.length(e.name)
-            tokens += e.tokens
-            positions += range(start, start + n)
-            row_seq += [i] * n
-            previous += [cache.last_token(e.name), *e.tokens[:-1]]
-            rows += n
-            cu.append(rows)
-            starts.append(start)
-            lengths.append(start + n)
-            slots.append(cache.slot(e.name))
+    def _fill(self, layout: _Layout, host: torch.Tensor, portions) -> None:
+        """A step's metadata into its buffer; sequences behind the portions are padding."""
+        cache, kept, records = self.cache, [], array("q")
+        for p in portions:
+            tokens = p.tokens if type(p.tokens) is array else array("q", p.tokens)
+            kept.append(tokens)
+            records.extend((tokens.buffer_info()[0], len(tokens), cache.length(p.name), cache.slot(p.name), int(cache.last_token(p.name))))
             for plane in range(layout.planes):
-                pages = cache.pages(e.name, plane)[:layout.width]
-                v["tables"][plane, i, :len(pages)] = torch.tensor(pages, dtype=torch.int32)
-        for _ in range(layout.sequences - len(entries)):     # padding sequences of one row
-            tokens.append(0); positions.append(0); row_seq.append(-1); previous.append(-1); starts.append(0); lengths.append(0)
-            slots.append(cache.dummy_slot)
-            cu.append(cu[-1] + 1)
-        for name, values in (("tokens", tokens), ("positions", positions), ("row_seq", row_seq), ("previous", previous), ("cu", cu), ("starts", starts),
-                             ("lengths", lengths), ("slots", slots)):
-            v[name].copy_(torch.tensor(values))
-        base = cu[layout.short]
-        v["long_cu"].copy_(torch.tensor([c - base for c in cu[layout.short:]]))
+                records.extend(cache.page_words(p.name, plane).buffer_info())
+        at = array("q", [where.start for where in layout.at.values()])
+        _capi.check(_capi.load().rlt_step_metadata(host.data_ptr(), at.buffer_info()[0], records.buffer_info()[0], len(portions), layout.sequences,
+                                                   layout.planes, layout.width, layout.short, layout.rows, cache.dummy_slot), "step")
 
     def _host_buffer(self, size: int) -> torch.Tensor:
         # from the caching host allocator: reused only after the copy that reads it has run
-        return torch.zeros(size, dtype=torch.int32, pin_memory=self.device.type == "cuda")
+        return torch.empty(size, dtype=torch.int32, pin_memory=self.device.type == "cuda")
+
+    def _indices(self, values: list) -> torch.Tensor:
+        """int64 indices on the device, without waiting for what is queued there."""
+        host = torch.tensor(values, dtype=torch.int64)
+        if self.device.type == "cuda":
+            host = host.pin_memory()
+        return host.to(self.device, non_blocking=True)
 
     def _batch(self, ordered) -> StepBatch:
         """The uploaded metadata of entries whose pages are reserved; short portions come first."""
@@ -280,7 +298,7 @@ class Engine:
         wanted = [first[e.name] + w for e in entries for w in e.want]
         if not wanted:
             return torch.empty(0, self.model.vocab_size, device=self.device)
-        return self.model.step_logits(hidden, torch.tensor(wanted, dtype=torch.int64, device=self.device))
+        return self.model.step_logits(hidden, self._indices(wanted))
 
     # ---- decode steps from graphs --------------------------------------------------------------
     def _bucket(self, n: int) -> int:

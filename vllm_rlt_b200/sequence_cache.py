@@ -10,6 +10,7 @@ sequence ignores what its slot holds.
 
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 
 import torch
@@ -49,7 +50,7 @@ class CacheFull(RuntimeError):
 @dataclass
 class _Sequence:
     slot: int
-    pages: list            # one list of page ids per plane
+    pages: list            # one array of page ids per plane
     length: int = 0        # tokens stored
     last: int = -1         # the last of them
 
@@ -108,10 +109,19 @@ class SequenceCache:
     def length(self, name) -> int:
         return self._sequences[name].length
 
+    def extent(self, name) -> tuple:
+        """Tokens stored and pages held per plane; nothing of a sequence that is not admitted."""
+        sequence = self._sequences.get(name)
+        return (sequence.length, len(sequence.pages[0])) if sequence else (0, 0)
+
     def slot(self, name) -> int:
         return self._sequences[name].slot
 
     def pages(self, name, plane: int = 0) -> list:
+        return self._sequences[name].pages[plane].tolist()
+
+    def page_words(self, name, plane: int = 0) -> array:
+        """The same as the 32-bit words of a page table's row; the sequence's own, to be read only."""
         return self._sequences[name].pages[plane]
 
     def pages_for(self, tokens: int) -> int:
@@ -123,7 +133,7 @@ class SequenceCache:
             raise ValueError(f"sequence {name!r} is already admitted")
         if not self._free_slots:
             raise CacheFull(f"all {self.max_sequences} sequence slots are taken")
-        self._sequences[name] = _Sequence(self._free_slots.pop(), [[] for _ in range(self.spec.planes)])
+        self._sequences[name] = _Sequence(self._free_slots.pop(), [array("i") for _ in range(self.spec.planes)])
 
     def reserve(self, name, tokens: int) -> None:
         """Pages for the sequence's first `tokens` tokens on every plane."""
@@ -131,8 +141,9 @@ class SequenceCache:
         need = max(-(-tokens // self.block) - len(sequence.pages[0]), 0)
         if need * self.spec.planes > len(self._free_pages):
             raise CacheFull(f"{need * self.spec.planes} pages asked, {len(self._free_pages)} free")
-        for pages in sequence.pages:
-            pages.extend(self._free_pages.pop() for _ in range(need))
+        for pages in sequence.pages if need else ():
+            pages.extend(self._free_pages[:-need - 1:-1])
+            del self._free_pages[-need:]
 
     def last_token(self, name) -> int:
         """The last stored token, -1 before the first (-1 too when `advance` was not told)."""
