@@ -262,6 +262,19 @@ def test_prompt_attention_over_expanded_latents(heads, dim, rot, vdim, window, p
     close(got, want, torch.bfloat16, 2.0)
 
 
+def test_windowed_prompt_attention_is_the_same_every_time():
+    """Late first copies (nothing of the keys in L2): the second tile of a pair starts behind the first and must not take a slot before its round."""
+    rows, heads, window, g = 8191, 16, 1024, torch.Generator(device="cuda").manual_seed(5)
+    normal = lambda *shape: torch.randn(shape, generator=g, device="cuda", dtype=torch.bfloat16)
+    q, kv, shared, flush = normal(rows, heads, 192), normal(rows, heads * 256), normal(rows, 64), torch.empty(2 ** 26, device="cuda")
+    ranges, outs = KeyRanges.of([(0, rows)], window, torch.device("cuda")), []
+    for _ in range(20):
+        flush.zero_()
+        outs.append(torch.empty(rows, heads, 128, dtype=torch.bfloat16, device="cuda"))
+        rlt.latent_prompt_attention(q, kv, shared, outs[-1], 128, ranges, 192 ** -0.5, window)
+    assert all(torch.equal(out, outs[0]) for out in outs)
+
+
 @pytest.mark.parametrize("heads,dim,rot,vdim", [(2, 128, 64, 128), (2, 64, 32, 80)])
 @pytest.mark.parametrize("window", [16, 64, 130, 200])
 def test_prompt_rows_find_a_key_just_inside_the_window_and_none_outside(heads, dim, rot, vdim, window):

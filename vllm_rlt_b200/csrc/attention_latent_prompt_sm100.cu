@@ -12,8 +12,8 @@
 //   warps 8, 9         issue the Q K^T products of tile 0 / 1,     warps 10, 11  the P V products
 //   warp 12            the copies: Q once, then the stages
 // Scores and probabilities have TMEM columns of their own, so S(j + 1) runs under the softmax of S(j), and O += P(j) V(j) follows
-// when P(j) is stored.  A tile walks the stages that hold a key some row of it sees: with a window the two tiles start at different
-// ones, and a stage that only one of them reads is released by the other's hand.
+// when P(j) is stored.  A tile walks the stages that hold a key some row of it sees: with a window tile 1 starts behind tile 0 and lets the
+// stages in front of it pass, and a stage behind the end of tile 0 is released by tile 1 for both.
 // TMEM columns: S0 0..63, P0 64..95 | S1 96..159, P1 160..191 | O0 256..383 | O1 384..511.
 #include "latent_attention.cuh"
 #include "layer_math.cuh"
@@ -35,7 +35,7 @@ struct PromptShared {
   static constexpr int kStageBytes = (kK + kR + kV) * kBlock;
   static constexpr int kFit = (220 * 1024 - 2 * (kK + kR) * kQBlock) / kStageBytes;
   static constexpr int kStages = kFit < 6 ? kFit : 6;
-  static_assert(kStages > kRows / kKeys, "tile 1 may start kRows keys behind tile 0: its first stage must be in the ring's first round");
+  static_assert(kStages >= 2, "copies run ahead of the products");
   unsigned char q[2][kK + kR][kQBlock];     // [tile][block][row][64], 128-byte swizzle; the output's staging rows in the end
   unsigned char k[kStages][kK + kR][kBlock];
   unsigned char v[kStages][kV][kBlock];
@@ -63,6 +63,13 @@ __device__ __forceinline__ bool issue_products(PromptShared<kK, kR, kV>& sm, uin
   constexpr int kStages = PromptShared<kK, kR, kV>::kStages;
   const uint32_t s_col = tmem + t * kTileCols, o_col = tmem + kColO + t * kRows;
   if (kScores && mine.begin < mine.end && !__all_sync(0xffffffffu, mbar_wait(smem_u32(&sm.full_q), 0))) return true;
+  // Stages in front of the tile's first are seen and given back as well: skipped, the parity of a ring slot's second round would read as
+  // complete while its first copy is still on the way, and the product would take whatever lies there.
+  for (int j = 0; j < mine.begin; ++j) {
+    if (!__all_sync(0xffffffffu, mbar_wait(smem_u32(kScores ? &sm.full_k[j % kStages] : &sm.full_v[j % kStages]), (j / kStages) & 1))) return true;
+    if (elect_one()) mbar_arrive(smem_u32(kScores ? &sm.free_k[j % kStages] : &sm.free_v[j % kStages]));
+    __syncwarp();
+  }
   const uint64_t q_desc = umma_desc(smem_u32(&sm.q[t][0][0]), 16, 1024);
   for (int j = mine.begin; j < mine.end; ++j) {
     const int i = j - mine.begin, stage = j % kStages;
@@ -76,7 +83,7 @@ __device__ __forceinline__ bool issue_products(PromptShared<kK, kR, kV>& sm, uin
     }
     if (!__all_sync(0xffffffffu, ok)) return true;
     tcgen05_after_sync();
-    const bool alone = j < other.begin || j >= other.end;       // the other tile does not read this stage
+    const bool alone = j >= other.end;            // the other tile is through
     if (kScores) {
       const uint64_t k_desc = umma_desc(smem_u32(&sm.k[stage][0][0]), 16, 1024);
       if (elect_one()) {
