@@ -174,6 +174,28 @@ def test_row_bits_do_not_depend_on_group_membership(kernel):
     assert torch.equal(shuffled, grouped[perm])
 
 
+@pytest.mark.parametrize("sequences", [1, 33, 1030])
+def test_packed_plan_gives_the_bits_of_single_rows(kernel, sequences):
+    # Sequences are searched 32 at a time, groups of up to 1024 rows are kept between the two passes: one and several rounds of both, with
+    # sequences without rows and without keys.
+    g = torch.Generator().manual_seed(sequences)
+    rows_per = torch.randint(0, 4, (sequences,), generator=g).tolist()
+    rows_per[-1] = 3
+    contexts = [max(n, 1) + int(torch.randint(0, 40, (1,), generator=g)) for n in rows_per]
+    contexts[0] = 0 if sequences > 1 else 700
+    pool = make_pool([max(c, 1) for c in contexts], kv_heads=16, head_dim=128, block=16, dtype=torch.bfloat16, seed=sequences)
+    cu = torch.tensor([0] + rows_per).cumsum(0).to(torch.int32)
+    rows = int(cu[-1])
+    q = (torch.randn(rows, 16, 128, generator=g) * 0.5).bfloat16()
+    lengths = torch.tensor(contexts, dtype=torch.int32)
+    packed = run_gpu(kernel, q, pool["key_pool"], pool["value_pool"], 0, pool["tables"], lengths, cu)
+    owner = torch.repeat_interleave(torch.arange(sequences), torch.tensor(rows_per))
+    single = (lengths[owner] - cu[1:][owner] + torch.arange(rows) + 1).clamp_min(0).to(torch.int32)
+    order = torch.randperm(rows, generator=g)
+    alone = run_gpu(kernel, q[order], pool["key_pool"], pool["value_pool"], 0, pool["tables"][owner[order]], single[order])
+    assert torch.equal(packed[order], alone)
+
+
 def test_shared_plan_runs_every_layer_with_one_plan(kernel):
     # One plan, many runs: every layer of a pass shares block tables and lengths.  The result of
     # each layer must equal the self-planned call bit for bit, including zero-length rows and
