@@ -473,6 +473,7 @@ constexpr int kMergeWarps = 4;
 template <bool kBF16>
 __global__ void __launch_bounds__(kMergeWarps * 32)
 merge_kernel(AttentionArgs a, Workspace ws) {
+  grid_dependency_wait();
   using T = typename std::conditional<kBF16, __nv_bfloat16, __half>::type;
   const int lane = threadIdx.x & 31;
   const int64_t pair = static_cast<int64_t>(blockIdx.x) * kMergeWarps + (threadIdx.x >> 5);
@@ -545,6 +546,7 @@ verify_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   __syncwarp();
+  grid_dependency_wait();   // plan, queries and pages belong to the kernels before until here; 4 us of a round come up under their tails
   // Rows of length zero: zeros, their block table is never read.
   {
     const unsigned zero_rows = ws.header->zero_rows;
@@ -888,12 +890,11 @@ int launch_main(const CUtensorMap& k_map, const CUtensorMap& v_map, const Attent
   const float scale_log2 = log2_scale(a);
   auto kernel = verify_attention_kernel<kBF16, kWarps, kStages, kCopies, kTerms>;
   RLT_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  kernel<<<sm_count, kWarps * 32, smem, stream>>>(k_map, v_map, a, ws, scale_log2, k_first ? 1 : 0);
-  int status = launch_status("verify_attention_kernel");
+  const int status = launch_dependent("verify_attention_kernel", kernel, dim3(static_cast<unsigned>(sm_count)), dim3(kWarps * 32), smem, stream, k_map, v_map, a, ws,
+                                      scale_log2, k_first ? 1 : 0);
   if (status != RLT_OK || ws.max_chunks < 2) return status;  // no context can span two chunks
   const int64_t pairs = static_cast<int64_t>(a.rows) * a.q_heads;
-  merge_kernel<kBF16><<<static_cast<unsigned>((pairs + kMergeWarps - 1) / kMergeWarps), kMergeWarps * 32, 0, stream>>>(a, ws);
-  return launch_status("merge_kernel");
+  return launch_dependent("merge_kernel", merge_kernel<kBF16>, dim3(static_cast<unsigned>((pairs + kMergeWarps - 1) / kMergeWarps)), dim3(kMergeWarps * 32), 0, stream, a, ws);
 }
 
 }  // namespace
