@@ -138,3 +138,17 @@ def test_layer_kernels_validate_their_arguments():
         rlt.rope_kv_write(q, q, q, q[:, 0], q[:, 0], torch.zeros(1, 4, 2, 7, device="cuda"),
                           torch.zeros(1, 4, 2, 7, device="cuda"), torch.zeros(2, dtype=torch.int64, device="cuda"),
                           torch.zeros(2, dtype=torch.int64, device="cuda"))
+
+
+@pytest.mark.parametrize("dtype, hidden", [(torch.bfloat16, 2048), (torch.float16, 2048), (torch.float32, 1024)])
+@pytest.mark.parametrize("rows", [1024, 1027])
+def test_norms_of_many_rows_give_the_bits_of_few(dtype, hidden, rows):
+    # A prompt's rows take a warp each, fewer than 1024 a CTA each.
+    g = torch.Generator(device="cuda").manual_seed(rows)
+    normal = lambda *shape: torch.randn(shape, generator=g, device="cuda").to(dtype)
+    x, residual, w, w2 = normal(rows, hidden), normal(rows, hidden), normal(hidden), normal(hidden)
+    halves = [slice(0, rows // 2), slice(rows // 2, rows)]
+    for res, second in ((None, None), (residual, None), (residual, w2), (None, w2)):
+        outs = [rlt.sandwich_norm(x[s], w, 1e-6, None if res is None else res[s], second) for s in (slice(None), *halves)]
+        for whole, *parts in zip(*outs):
+            assert whole is None or torch.equal(whole, torch.cat(parts))
