@@ -440,6 +440,21 @@ def test_expert_products_of_pairs_of_ctas(inner, outer, counts):
     close(got, want.cpu(), torch.bfloat16, 2.0)
 
 
+@pytest.mark.parametrize("inner", [64, 384, 400])
+@pytest.mark.parametrize("counts", [[97], [300], [0, 700], [257, 256, 255, 0, 1]])
+def test_pairs_of_ctas_end_with_every_stage_given_back(inner, counts):
+    """Fewer copies than stages, a whole round of them and one more, on pairs that have a tile and on pairs that have none: each launch waits for
+    what gives its stages back, and the next one on the same multiprocessors computes the same bits."""
+    g = torch.Generator().manual_seed(inner)
+    x = torch.randn(sum(counts), inner, generator=g).bfloat16().cuda()
+    w = (torch.randn(len(counts), 392, inner, generator=g) / inner ** 0.5).bfloat16().cuda()
+    per = torch.tensor(counts, dtype=torch.int32, device="cuda")
+    outs = [rlt.expert_gemm(x, w, per) for _ in range(8)]
+    want = torch.cat([rows.double() @ w[e].double().T for e, rows in enumerate(x.split(counts))])
+    close(outs[0], want.cpu(), torch.bfloat16, 2.0)
+    assert all(torch.equal(out, outs[0]) for out in outs)
+
+
 def test_the_mamba_scan_still_takes_its_own_decays():
     """Both forms of the recurrence share their kernels: driven by step sizes it is what it was."""
     g = torch.Generator().manual_seed(2)

@@ -171,6 +171,11 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
           if (++stage == kStages) { stage = 0; parity ^= 1u; }
         }
       }
+      // The commits that give the last stages back arrive on their own time, a pair's in both CTAs: wait for them before the memory goes.
+      for (int s = 0; s < kStages && !failed; ++s) {
+        failed = !mbar_wait(smem_u32(&sm.empty[stage]), parity);
+        if (++stage == kStages) { stage = 0; parity ^= 1u; }
+      }
     }
     __syncwarp();
   } else if (warp == 1) {
@@ -256,7 +261,7 @@ expert_gemm_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_const
   if (failed && lane == 0) atomicOr(g.error, 1u);
   tcgen05_before_sync();
   __syncthreads();
-  if constexpr (kCtas > 1) cluster_sync();         // neither CTA leaves while the other may still reach its memory
+  if constexpr (kCtas > 1) cluster_sync();         // neither CTA leaves while the other's copies, products and arrivals may reach its memory
   if (warp == 1) free_tmem<kCtas>(tmem, kColumns);
 }
 
