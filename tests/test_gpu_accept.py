@@ -227,6 +227,35 @@ def test_filters_where_a_selection_changes_its_way_match_oracle_bit_for_bit(voca
         assert torch.equal(tokens.cpu(), oracle.sample_rows(logits.contiguous(), temperature, uniforms, top_k, top_p)[0])
 
 
+@pytest.mark.parametrize("vocab,dtype", [(49152, torch.float32), (20001, torch.bfloat16), (3000, torch.float32)])
+def test_filters_of_rows_that_a_histogram_has_to_divide_again(vocab, dtype):
+    """Rows whose bulk is narrow beside its distance from a peak or from masked tokens, bands of their own, ties in the thousands and values next
+    to each other: the steps of the first histogram, of the next ones, and what no step tells apart."""
+    g = torch.Generator().manual_seed(vocab)
+    x = torch.randn(10, vocab, generator=g)
+    x[0] *= 1e-3
+    x[1] = x[1] * 1e-3 - 8
+    x[1, 7] = 0.0                                       # the bulk in one step of the first histogram
+    x[2] *= 1e-3
+    x[2, ::2] = -1e4
+    x[3] = (x[3] > 0.5).float() * 2.0                   # two values
+    x[4] = 0.0
+    x[5] = torch.where(x[5] > 0, x[5] * 1e-6, 5 + x[5] * 1e-6)          # two bands
+    x[6] *= 1e-42                                       # denormals
+    x[7] = 1.0 + (torch.rand(vocab, generator=g) * 8).floor() * 2 ** -23 if dtype == torch.float32 else 1.0
+    x[8] *= 300
+    x[8, 5] = 3e4
+    x[9, vocab // 2:] = float("-inf")
+    logits = x.to(dtype)
+    cuda, ones = logits.cuda(), torch.ones(10)
+    for top_k, top_p, temperature in ((-1, 0.95, 0.8), (-1, 0.3, 1.0), (vocab - 3, 1.0, 1.0), (1500, 0.5, 1.0), (2500, 0.9999, 1e-3), (50, 0.95, 1e3), (300, 0.7, 1.0)):
+        k, p, t = torch.full((10,), top_k, dtype=torch.int32), ones * top_p, ones * temperature
+        want = _oracle_probabilities(logits, t, k, p)
+        got, status = rlt.probabilities(cuda, t.cuda(), k.cuda(), p.cuda())
+        assert not status.any()
+        assert torch.equal(got.cpu(), want), (top_k, top_p, [r for r in range(10) if not torch.equal(got[r].cpu(), want[r])])
+
+
 def test_probabilities_reject_greedy_and_bad_rows():
     logits = torch.randn(3, 64)
     logits[2, 5] = float("nan")

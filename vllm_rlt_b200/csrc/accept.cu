@@ -265,95 +265,202 @@ __device__ __forceinline__ float block_cut_sum(const T* __restrict__ row, int vo
 // pass), several CTAs per SM:
 //   candidates   top-k up to a token per thread: at least k tokens reach the k-th largest of the threads' own maxima, so the few
 //                tokens at or above that value (70 for k = 50 of 49 152) hold the whole answer, and top-p inside it.
-//   buckets      every other filter: a histogram of weight over m - t in steps of 1/64 finds the step in which the running weight
-//                first exceeds the limit; its tokens are the candidates.
-//   digits       rows whose candidates do not fit (mass ties): a radix select over four 8-bit digits of the order key.
-// 128 requests of 5 rows of 49 152 fp32 logits, half of them with top-k 50 and top-p 0.95: the digits alone, over a row copied
-// to shared memory by one CTA per SM, took 595 us; this takes 141 us.
+//   buckets      every other filter: a histogram of weight over the distance from the maximum finds the step in which the running
+//                weight first exceeds the limit; its tokens are the candidates, or are divided once more where they do not fit.
+//                Steps are as wide as the row is spread, so a flat row fills as many of them as a peaked one.
+//   digits       what is left (values that a step cannot tell apart): a radix select over four 8-bit digits of the order key.
+// 128 requests of 5 rows of 49 152 fp32 logits, half of them with top-k 50 and top-p 0.95: 107 us.  One row of 49 152, top-p 0.95 alone: 74 us of
+// which 37 are the draw without a filter; 87 us where all logits lie within a hundredth of each other, 206 us where all are equal.  Top-k
+// 50 of it: 23 us with one warp ranking the 70 candidates, 42 with the whole CTA, whose every bit of the key costs two barriers.
 constexpr int kCandidates = 2048;
 constexpr int kBuckets = 2048;
+constexpr int kWarpCandidates = 128;        // up to this many are ranked by one warp, from registers
 
 struct SelectScratch {
   union {
-    struct {                                // candidates, and the digits' histogram
+    struct {                                // candidates
       unsigned long long weight[kCandidates];
       uint32_t key[kCandidates];
       int index[kCandidates];
     };
     unsigned long long bucket[kBuckets];
-    struct {
-      unsigned long long mass[256];
-      unsigned int count[256];
-    };
   };
+  unsigned long long mass[256];             // the digits' histogram
+  unsigned int count[256];
   unsigned long long above;
   int digit;
   int found;
   int listed;
+  uint32_t lowest, highest;                 // keys of the candidates
+  Cut cut;
   int warp_counts[32];
 };
 
-__device__ __forceinline__ int bucket_of(float t, float m) {
-  const float d = RLT_SUB(m, t);
-  return d < 31.0f ? max(static_cast<int>(d * 64.0f), 0) : kBuckets - 1;
+// Sums of lanes' weights that are below 2^44 together per lane: two 22-bit halves, so that 32 of them fit a word.
+__device__ __forceinline__ unsigned long long sum_weights(unsigned lanes, unsigned long long w) {
+  const unsigned low = __reduce_add_sync(lanes, static_cast<unsigned>(w & 0x3fffffu));
+  const unsigned high = __reduce_add_sync(lanes, static_cast<unsigned>(w >> 22));
+  return (static_cast<unsigned long long>(high) << 22) + low;
 }
 
-// Adds a token to the candidates; those that do not fit are only counted.
-__device__ __forceinline__ void list_token(SelectScratch& h, uint32_t key, int index) {
-  const int at = atomicAdd(&h.listed, 1);
-  if (at < kCandidates) { h.key[at] = key; h.index[at] = index; }
+// Adds a token to the candidates, one atomic for the lanes that are here together; those that do not fit are only counted.
+__device__ __forceinline__ void list_token(SelectScratch& h, uint32_t key, int index, unsigned long long weight) {
+  const unsigned here = __activemask();
+  const int lane = threadIdx.x & 31, first = __ffs(here) - 1;
+  int at = 0;
+  if (lane == first) at = atomicAdd(&h.listed, __popc(here));
+  at = __shfl_sync(here, at, first) + __popc(here & ((1u << lane) - 1u));
+  if (at < kCandidates) { h.key[at] = key; h.index[at] = index; h.weight[at] = weight; }
 }
 
-// The cut among n listed candidates with their weights, `above` being the weight of the tokens ranked before all of them.
-// A candidate whose weight no longer counts has weight 0 and key 0.  The running weight must exceed the limit inside the list.
-template <int kThreads>
-__device__ __forceinline__ Cut list_select(SelectScratch& h, int n, unsigned long long above, unsigned long long limit, Cut outer,
-                                           unsigned long long* scratch) {
-  auto weight_where = [&](auto&& counts) {
-    unsigned long long sum = 0ull;
-    for (int j = threadIdx.x; j < n; j += kThreads)
-      if (counts(j)) sum += h.weight[j];
-    return block_sum<kThreads>(sum, scratch);
-  };
-  uint32_t key = 0u;                        // the largest key for which the weight of all tokens from it on exceeds the limit
-  for (int bit = 31; bit >= 0; --bit) {
-    const uint32_t next = key | (1u << bit);
-    if (above + weight_where([&](int j) { return h.key[j] >= next; }) > limit) key = next;
-  }
-  const unsigned long long before = above + weight_where([&](int j) { return h.key[j] > key; });
-  int ties = 0;
-  unsigned long long each = 0ull;
-  for (int j = threadIdx.x; j < n; j += kThreads)
-    if (h.key[j] == key) { ++ties; each = h.weight[j]; }
-  ties = static_cast<int>(block_sum<kThreads>(static_cast<unsigned long long>(ties), scratch));
-  each = block_max<kThreads>(each, scratch);
-  const unsigned long long keep = (limit - before) / each + 1ull;
-  if (keep >= static_cast<unsigned long long>(ties)) return Cut{key, key == outer.key ? outer.limit : 0x7fffffff};
-  int index = 0;                            // the largest index with fewer than `keep` of the tied tokens before it
-  for (int bit = 30; bit >= 0; --bit) {
-    const int next = index | (1 << bit);
-    unsigned long long count = 0ull;
-    for (int j = threadIdx.x; j < n; j += kThreads) count += h.key[j] == key && h.index[j] < next;
-    if (block_sum<kThreads>(count, scratch) < keep) index = next;
-  }
-  return Cut{key, index};
+// Adds to a bucket by atomics on its two words, the low one's carry going into the high one: 32-bit adds are done by the memory itself, a 64-bit
+// one retries for as long as other lanes get in between, which takes 40 times as long where the tokens of a row share a bucket.
+__device__ __forceinline__ void bucket_add(SelectScratch& h, int bucket, unsigned long long w) {
+  unsigned* word = reinterpret_cast<unsigned*>(&h.bucket[bucket]);
+  const unsigned low = static_cast<unsigned>(w), before = atomicAdd(word, low);
+  const unsigned high = static_cast<unsigned>(w >> 32) + (before + low < low ? 1u : 0u);
+  if (high != 0u) atomicAdd(word + 1, high);
 }
-
-// One shared-memory atomic per distinct digit in the warp: lanes with the same digit find each
-// other with match.any and add their weights with two integer warp reductions (a weight is below
-// 2^41: 20 low and 21 high bits, so 32 of them cannot overflow a 32-bit partial sum).  The leading
-// byte of the key has only a few populated values, so plain per-lane atomics would serialise.
+// One shared-memory atomic per distinct digit in the warp: lanes with the same digit find each other with match.any and add their weights
+// (below 2^41) first.  The leading byte of the key has only a few populated values.
 template <bool kByMass>
-__device__ __forceinline__ void hist_add(SelectScratch& h, int bucket, unsigned long long w, bool valid) {
+__device__ __forceinline__ void digit_add(SelectScratch& h, int digit, unsigned long long w, bool valid) {
   const int lane = threadIdx.x & 31;
-  const unsigned peers = __match_any_sync(0xffffffffu, valid ? bucket : 0x7fff);
+  const unsigned peers = __match_any_sync(0xffffffffu, valid ? digit : 0x7fff);
   const bool leader = valid && lane == __ffs(peers) - 1;
   if (kByMass) {
-    const unsigned low = __reduce_add_sync(peers, static_cast<unsigned>(w & 0xfffffu));
-    const unsigned high = __reduce_add_sync(peers, static_cast<unsigned>(w >> 20));
-    if (leader) atomicAdd(&h.mass[bucket], (static_cast<unsigned long long>(high) << 20) + low);
+    const unsigned long long sum = sum_weights(peers, w);
+    if (leader) atomicAdd(&h.mass[digit], sum);
   }
-  if (leader) atomicAdd(&h.count[bucket], static_cast<unsigned int>(__popc(peers)));
+  if (leader) atomicAdd(&h.count[digit], static_cast<unsigned int>(__popc(peers)));
+}
+
+// The key at which the running weight of `count` items, ranked by key from the largest on and starting at `above`, first exceeds the limit:
+// four passes over 8-bit digits, most significant first.  item(i, &key, &weight) says whether item i counts.  False where the limit is never
+// exceeded.  `ties` items have the key and a weight of `each`; those before them add up to `before`.
+struct Crossing { uint32_t key; unsigned int ties; unsigned long long each, before; };
+template <int kThreads, bool kByMass, typename Item>
+__device__ __forceinline__ bool digit_select(SelectScratch& h, int count, unsigned long long above, unsigned long long limit, Crossing* at, Item item) {
+  uint32_t prefix = 0u;
+  for (int pass = 0; pass < 4; ++pass) {
+    const int shift = 24 - 8 * pass;
+    __syncthreads();
+    for (int i = threadIdx.x; i < 256; i += kThreads) { h.mass[i] = 0ull; h.count[i] = 0u; }
+    __syncthreads();
+    for (int base = 0; base < count; base += kThreads) {
+      const int i = base + static_cast<int>(threadIdx.x);
+      uint32_t key = 0u;
+      unsigned long long w = 0ull;
+      const bool valid = i < count && item(i, &key, pass, prefix >> (shift + 7) >> 1, &w);
+      digit_add<kByMass>(h, static_cast<int>((key >> shift) & 255u), w, valid);
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      // lane l scans digits 255 - 8l down to 248 - 8l
+      const int lane = threadIdx.x, hi = 255 - 8 * lane;
+      unsigned long long local = 0ull;
+#pragma unroll
+      for (int j = 0; j < 8; ++j) local += kByMass ? h.mass[hi - j] : static_cast<unsigned long long>(h.count[hi - j]);
+      unsigned long long inc = local;
+#pragma unroll
+      for (int x = 1; x < 32; x <<= 1) {
+        const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, x);
+        if (lane >= x) inc += o;
+      }
+      const unsigned crossing = __ballot_sync(0xffffffffu, above + inc > limit);
+      if (crossing == 0u) {
+        if (lane == 0) h.digit = -1;
+      } else if (lane == __ffs(crossing) - 1) {
+        unsigned long long acc = above + inc - local;
+        int digit = hi;
+        for (int j = 0; j < 8; ++j) {
+          const unsigned long long wd = kByMass ? h.mass[hi - j] : static_cast<unsigned long long>(h.count[hi - j]);
+          digit = hi - j;
+          if (acc + wd > limit) break;
+          acc += wd;
+        }
+        h.digit = digit;
+        h.above = acc;
+      }
+    }
+    __syncthreads();
+    if (h.digit < 0) return false;
+    prefix |= static_cast<uint32_t>(h.digit) << shift;
+    above = h.above;
+  }
+  at->key = prefix;
+  at->before = above;
+  at->ties = h.count[prefix & 255u];
+  at->each = kByMass ? h.mass[prefix & 255u] / at->ties : 1ull;
+  return true;
+}
+
+// The cut among n listed candidates, `above` being the weight of the tokens ranked before all of them.  A candidate that no longer counts
+// has weight 0 and key 0.  The running weight must exceed the limit inside the list.
+template <int kThreads>
+__device__ __noinline__ Cut list_select(SelectScratch& h, int n, unsigned long long above, unsigned long long limit, Cut outer) {
+  if (n <= kWarpCandidates) {
+    __syncthreads();
+    if (threadIdx.x < 32) {
+      constexpr int kOwn = kWarpCandidates / 32;
+      const int lane = threadIdx.x;
+      uint32_t own_key[kOwn];
+      unsigned long long own[kOwn];
+#pragma unroll
+      for (int i = 0; i < kOwn; ++i) {
+        own_key[i] = lane + 32 * i < n ? h.key[lane + 32 * i] : 0u;
+        own[i] = lane + 32 * i < n ? h.weight[lane + 32 * i] : 0ull;
+      }
+      auto weight_from = [&](uint32_t from) {
+        unsigned long long sum = 0ull;
+#pragma unroll
+        for (int i = 0; i < kOwn; ++i) sum += own_key[i] >= from ? own[i] : 0ull;
+        return sum_weights(0xffffffffu, sum);
+      };
+      uint32_t key = 0u;                    // the largest key for which the weight of all tokens from it on exceeds the limit
+      for (int bit = 31; bit >= 0; --bit)
+        if (above + weight_from(key | (1u << bit)) > limit) key |= 1u << bit;
+      const unsigned long long before = above + weight_from(key + 1u);
+      int ties = 0;
+      unsigned long long each = 0ull;
+#pragma unroll
+      for (int i = 0; i < kOwn; ++i) {
+        const unsigned tied = __ballot_sync(0xffffffffu, own_key[i] == key);
+        if (tied != 0u) each = __shfl_sync(0xffffffffu, own[i], __ffs(tied) - 1);
+        ties += __popc(tied);
+      }
+      const unsigned long long keep = (limit - before) / each + 1ull;
+      int index = key == outer.key ? outer.limit : 0x7fffffff;
+      if (keep < static_cast<unsigned long long>(ties)) {
+        index = 0;                          // the largest index with fewer than `keep` of the tied tokens before it
+        for (int bit = 30; bit >= 0; --bit) {
+          const int next = index | (1 << bit);
+          int smaller = 0;
+#pragma unroll
+          for (int i = 0; i < kOwn; ++i)
+            smaller += __popc(__ballot_sync(0xffffffffu, own_key[i] == key && h.index[lane + 32 * i] < next));
+          if (smaller < static_cast<int>(keep)) index = next;
+        }
+      }
+      if (lane == 0) h.cut = Cut{key, index};
+    }
+    __syncthreads();
+    return h.cut;
+  }
+  Crossing at;
+  digit_select<kThreads, true>(h, n, above, limit, &at, [&](int j, uint32_t* key, int pass, uint32_t chosen, unsigned long long* w) {
+    *key = h.key[j];
+    *w = h.weight[j];
+    return *key >> (31 - 8 * pass) >> 1 == chosen;
+  });
+  const unsigned long long keep = (limit - at.before) / at.each + 1ull;
+  if (keep >= at.ties) return Cut{at.key, at.key == outer.key ? outer.limit : 0x7fffffff};
+  Crossing last;                            // the keep-th of the tied tokens, smallest index first
+  digit_select<kThreads, false>(h, n, 0ull, keep - 1ull, &last, [&](int j, uint32_t* key, int pass, uint32_t chosen, unsigned long long* w) {
+    *key = 0xffffffffu - static_cast<uint32_t>(h.index[j]);
+    return h.key[j] == at.key && *key >> (31 - 8 * pass) >> 1 == chosen;
+  });
+  return Cut{at.key, static_cast<int>(0xffffffffu - last.key)};
 }
 
 // Index of the n-th (1-based) token in ascending index order with order key `key` inside `outer`.
@@ -388,135 +495,144 @@ __device__ __forceinline__ int block_nth_index(const T* __restrict__ row, int vo
   return h.found;
 }
 
+// The cut of the tokens in `outer`: by buckets; `inv` is 1 / z, `own` the thread's largest raw logit.
 template <typename T, int kThreads, bool kByMass>
-__device__ __forceinline__ Cut block_select(const T* __restrict__ row, int vocab, float temperature, float m,
-                                            float inv, Cut outer, unsigned long long limit, SelectScratch& h) {
-  uint32_t prefix = 0u;
-  unsigned long long above = 0ull;
-  for (int pass = 0; pass < 4; ++pass) {
-    const int shift = 24 - 8 * pass;
-    __syncthreads();
-    for (int i = threadIdx.x; i < 256; i += kThreads) { h.mass[i] = 0ull; h.count[i] = 0u; }
-    __syncthreads();
-    for (int base = 0; base < vocab; base += kThreads) {
-      const int v = base + static_cast<int>(threadIdx.x);
-      bool valid = false;
-      int bucket = 0;
-      unsigned long long w = 0ull;
-      if (v < vocab) {
-        const float t = scaled_logit(row, v, temperature);
-        const uint32_t key = rlt_order_key(t);
-        valid = rlt_in_support(key, v, outer.key, outer.limit) &&
-                (pass == 0 || (key >> (shift + 8)) == (prefix >> (shift + 8)));
-        bucket = static_cast<int>((key >> shift) & 255u);
-        if (kByMass && valid) w = rlt_fix_weight(rlt_draw_mass(rlt_expf(RLT_SUB(t, m)), inv));
-      }
-      hist_add<kByMass>(h, bucket, w, valid);
-    }
-    __syncthreads();
-    if (threadIdx.x < 32) {
-      // lane l scans digits 255 - 8l down to 248 - 8l
-      const int lane = threadIdx.x, hi = 255 - 8 * lane;
-      unsigned long long local = 0ull;
-#pragma unroll
-      for (int j = 0; j < 8; ++j) local += kByMass ? h.mass[hi - j] : static_cast<unsigned long long>(h.count[hi - j]);
-      unsigned long long inc = local;
-#pragma unroll
-      for (int x = 1; x < 32; x <<= 1) {
-        const unsigned long long o = __shfl_up_sync(0xffffffffu, inc, x);
-        if (lane >= x) inc += o;
-      }
-      const unsigned crossing = __ballot_sync(0xffffffffu, above + inc > limit);
-      if (crossing == 0u) {
-        if (lane == 0) h.digit = -1;
-      } else if (lane == __ffs(crossing) - 1) {
-        unsigned long long acc = above + inc - local;
-        int digit = hi;
-        for (int j = 0; j < 8; ++j) {
-          const unsigned long long wd = kByMass ? h.mass[hi - j] : static_cast<unsigned long long>(h.count[hi - j]);
-          digit = hi - j;
-          if (acc + wd > limit) break;
-          acc += wd;
-        }
-        h.digit = digit;
-        h.above = acc;
-      }
-    }
-    __syncthreads();
-    if (h.digit < 0) return outer;  // the whole of `outer` stays (its weight never exceeds the limit)
-    prefix |= static_cast<uint32_t>(h.digit) << shift;
-    above = h.above;
-  }
-  const unsigned int ties = h.count[prefix & 255u];
-  const unsigned long long each = kByMass ? h.mass[prefix & 255u] / ties : 1ull;
-  const unsigned long long keep = (limit - above) / each + 1ull;
-  __syncthreads();
-  if (keep >= ties) return Cut{prefix, prefix == outer.key ? outer.limit : 0x7fffffff};
-  return Cut{prefix, block_nth_index<T, kThreads>(row, vocab, temperature, prefix, outer,
-                                                  static_cast<unsigned int>(keep), h)};
-}
-
-// The cut by buckets (digits where the bucket's tokens do not fit the list); `inv` is 1 / z.
-template <typename T, int kThreads, bool kByMass>
-__device__ __forceinline__ Cut bucket_select(const T* __restrict__ row, int vocab, float temperature, float m, float inv, Cut outer,
+__device__ __forceinline__ Cut bucket_select(const T* __restrict__ row, int vocab, float temperature, float m, float inv, float own, Cut outer,
                                              unsigned long long limit, unsigned long long* scratch, SelectScratch& h) {
   constexpr int kOwn = kBuckets / kThreads;
-  const float floor = cut_floor(outer, temperature);
-  const auto weight = [&](float t) { return kByMass ? rlt_fix_weight(rlt_draw_mass(rlt_expf(RLT_SUB(t, m)), inv)) : 1ull; };
-  __syncthreads();
-  for (int i = threadIdx.x; i < kBuckets; i += kThreads) h.bucket[i] = 0ull;
-  if (threadIdx.x == 0) { h.digit = -1; h.listed = 0; }
-  __syncthreads();
-  for_row<T, kThreads, 2>(row, vocab, [&](float x, int v) {
-    if (x >= floor) {
-      const float t = RLT_DIV(x, temperature);
-      if (rlt_in_support(rlt_order_key(t), v, outer.key, outer.limit)) {
-        const unsigned long long w = weight(t);
-        if (w != 0ull) atomicAdd(&h.bucket[bucket_of(t, m)], w);
-      }
-    }
-  });
-  __syncthreads();
-  // thread i scans buckets kOwn * i ..
-  unsigned long long own[kOwn], local = 0ull;
-#pragma unroll
-  for (int j = 0; j < kOwn; ++j) { own[j] = h.bucket[kOwn * threadIdx.x + j]; local += own[j]; }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  unsigned long long before = local;
-#pragma unroll
-  for (int x = 1; x < 32; x <<= 1) {
-    const unsigned long long o = __shfl_up_sync(0xffffffffu, before, x);
-    if (lane >= x) before += o;
+  const auto weight = [&](float t) { return kByMass ? rlt_fix_weight(rlt_draw_mass(rlt_expf(RLT_SUB(t, m)), inv)) : 1ull; };
+  const auto cut_of_ties = [&](uint32_t key, unsigned long long ties, unsigned long long each, unsigned long long before) {
+    const unsigned long long keep = (limit - before) / each + 1ull;
+    if (keep >= ties) return Cut{key, key == outer.key ? outer.limit : 0x7fffffff};
+    return Cut{key, block_nth_index<T, kThreads>(row, vocab, temperature, key, outer, static_cast<unsigned int>(keep), h)};
+  };
+  if (vocab <= kCandidates) {               // the whole row fits the list
+    unsigned long long sum = 0ull;
+    __syncthreads();
+    for (int v = threadIdx.x; v < vocab; v += kThreads) {
+      const float t = scaled_logit(row, v, temperature);
+      const uint32_t key = rlt_order_key(t);
+      const unsigned long long w = rlt_in_support(key, v, outer.key, outer.limit) ? weight(t) : 0ull;
+      h.key[v] = w != 0ull ? key : 0u;
+      h.index[v] = v;
+      h.weight[v] = w;
+      sum += w;
+    }
+    if (block_sum<kThreads>(sum, scratch) <= limit) return outer;
+    return list_select<kThreads>(h, vocab, 0ull, limit, outer);
   }
-  if (lane == 31) scratch[warp] = before;
-  __syncthreads();
-  before -= local;
-  for (int w = 0; w < warp; ++w) before += scratch[w];
-  if (before <= limit && before + local > limit) {      // one thread at most
+  // Steps of the first histogram: four times the mean distance of the threads' own maxima, which the bulk of a row stays within however flat or
+  // peaked it is; masses end 28 below the maximum.
+  float distance = own == -INFINITY ? 0.0f : RLT_SUB(m, RLT_DIV(own, temperature)), holders = own == -INFINITY ? 0.0f : 1.0f;
 #pragma unroll
-    for (int j = 0; j < kOwn; ++j) {
-      if (h.digit < 0) {
-        if (before + own[j] > limit) { h.digit = kOwn * threadIdx.x + j; h.above = before; }
-        before += own[j];
+  for (int x = 16; x > 0; x >>= 1) {
+    distance += __shfl_xor_sync(0xffffffffu, distance, x);
+    holders += __shfl_xor_sync(0xffffffffu, holders, x);
+  }
+  __syncthreads();
+  if (lane == 0) scratch[warp] = static_cast<unsigned long long>(__float_as_uint(distance)) << 32 | __float_as_uint(holders);
+  __syncthreads();
+  distance = holders = 0.0f;
+  for (int w = 0; w < kThreads / 32; ++w) {
+    distance += __uint_as_float(static_cast<uint32_t>(scratch[w] >> 32));
+    holders += __uint_as_float(static_cast<uint32_t>(scratch[w]));
+  }
+  float range = 4.0f * distance / holders;
+  if (kByMass) range = fminf(range, 31.0f);
+  float top = m;
+  uint32_t low = 0u, high = 0xffffffffu;    // keys of the tokens that are being told apart
+  unsigned long long above = 0ull;          // weight of those ranked before them
+  for (int level = 0; level < 3; ++level) {
+    const float floor = fmaxf(cut_floor(outer, temperature), level == 0 ? -INFINITY : raw_floor(key_value(low), temperature));
+    const float scale = fminf((kBuckets - 2) / range, 0x1p120f);
+    // a step, never a smaller one for a smaller t
+    const auto bucket_of = [&](float t) { return static_cast<int>(fminf(fmaxf(RLT_SUB(top, t), 0.0f) * scale, kBuckets - 1.0f)); };
+    const auto among = [&](uint32_t key, int v) { return key >= low && key <= high && rlt_in_support(key, v, outer.key, outer.limit); };
+    __syncthreads();
+    for (int i = threadIdx.x; i < kBuckets; i += kThreads) h.bucket[i] = 0ull;
+    if (threadIdx.x == 0) { h.digit = -1; h.listed = 0; h.lowest = 0xffffffffu; h.highest = 0u; }
+    __syncthreads();
+    for_row<T, kThreads, 2>(row, vocab, [&](float x, int v) {
+      if (x >= floor) {
+        const float t = RLT_DIV(x, temperature);
+        if (among(rlt_order_key(t), v)) {
+          const unsigned long long w = weight(t);
+          if (kByMass) {
+            if (w != 0ull) bucket_add(h, bucket_of(t), w);
+          } else {
+            atomicAdd(reinterpret_cast<unsigned*>(&h.bucket[bucket_of(t)]), 1u);
+          }
+        }
+      }
+    });
+    __syncthreads();
+    // thread i scans buckets kOwn * i ..
+    unsigned long long held[kOwn], local = 0ull;
+#pragma unroll
+    for (int j = 0; j < kOwn; ++j) { held[j] = h.bucket[kOwn * threadIdx.x + j]; local += held[j]; }
+    unsigned long long before = local;
+#pragma unroll
+    for (int x = 1; x < 32; x <<= 1) {
+      const unsigned long long o = __shfl_up_sync(0xffffffffu, before, x);
+      if (lane >= x) before += o;
+    }
+    if (lane == 31) scratch[warp] = before;
+    __syncthreads();
+    before += above - local;
+    for (int w = 0; w < warp; ++w) before += scratch[w];
+    if (before <= limit && before + local > limit) {      // one thread at most
+#pragma unroll
+      for (int j = 0; j < kOwn; ++j) {
+        if (h.digit < 0) {
+          if (before + held[j] > limit) { h.digit = kOwn * threadIdx.x + j; h.above = before; }
+          before += held[j];
+        }
       }
     }
+    __syncthreads();
+    const int crossing = h.digit;
+    above = h.above;
+    if (crossing < 0) return outer;         // everything stays
+    uint32_t lowest = 0xffffffffu, highest = 0u;
+    for_row<T, kThreads>(row, vocab, [&](float x, int v) {
+      if (x >= floor) {
+        const float t = RLT_DIV(x, temperature);
+        const uint32_t key = rlt_order_key(t);
+        if (bucket_of(t) == crossing && among(key, v)) {
+          const unsigned long long w = weight(t);
+          if (w != 0ull) {
+            lowest = min(lowest, key);
+            highest = max(highest, key);
+            list_token(h, key, v, w);
+          }
+        }
+      }
+    });
+    lowest = __reduce_min_sync(0xffffffffu, lowest);
+    highest = __reduce_max_sync(0xffffffffu, highest);
+    if (lane == 0) { atomicMin(&h.lowest, lowest); atomicMax(&h.highest, highest); }
+    __syncthreads();
+    const int n = h.listed;
+    if (n <= kCandidates) return list_select<kThreads>(h, n, above, limit, outer);
+    low = h.lowest;
+    high = h.highest;
+    if (low == high) return cut_of_ties(low, n, weight(key_value(low)), above);
+    top = key_value(high);
+    range = RLT_SUB(top, key_value(low));
   }
-  __syncthreads();
-  const int crossing = h.digit;
-  const unsigned long long above = h.above;
-  if (crossing < 0) return outer;           // everything stays
-  for_row<T, kThreads>(row, vocab, [&](float x, int v) {
-    if (x >= floor) {
-      const float t = RLT_DIV(x, temperature);
-      const uint32_t key = rlt_order_key(t);
-      if (bucket_of(t, m) == crossing && rlt_in_support(key, v, outer.key, outer.limit)) list_token(h, key, v);
-    }
+  Crossing at;
+  const float floor = raw_floor(key_value(low), temperature);
+  digit_select<kThreads, kByMass>(h, vocab, above, limit, &at, [&](int v, uint32_t* key, int pass, uint32_t chosen, unsigned long long* w) {
+    const float x = Elem<T>::to_float(row[v]);
+    if (!(x >= floor)) return false;
+    const float t = RLT_DIV(x, temperature);
+    *key = rlt_order_key(t);
+    if (*key < low || *key > high || !rlt_in_support(*key, v, outer.key, outer.limit) || *key >> (31 - 8 * pass) >> 1 != chosen) return false;
+    *w = weight(t);
+    return *w != 0ull;
   });
-  __syncthreads();
-  const int n = h.listed;
-  if (n > kCandidates) return block_select<T, kThreads, kByMass>(row, vocab, temperature, m, inv, outer, limit, h);
-  for (int j = threadIdx.x; j < n; j += kThreads) h.weight[j] = weight(key_value(h.key[j]));
-  return list_select<kThreads>(h, n, above, limit, outer, scratch);
+  return cut_of_ties(at.key, at.ties, at.each, at.before);
 }
 
 // max, support and normaliser of the distribution Sampler.probabilities builds for one row
@@ -556,14 +672,13 @@ __device__ __forceinline__ RowNorm block_normalise(const T* __restrict__ row, in
       if (threadIdx.x == 0) h.listed = 0;
       __syncthreads();
       for_row<T, kThreads>(row, vocab, [&](float x, int v) {
-        if (x >= floor) list_token(h, rlt_order_key(RLT_DIV(x, temperature)), v);
+        if (x >= floor) list_token(h, rlt_order_key(RLT_DIV(x, temperature)), v, 1ull);
       });
       __syncthreads();
       listed = h.listed;
     }
     if (listed <= kCandidates) {
-      for (int j = threadIdx.x; j < listed; j += kThreads) h.weight[j] = 1ull;
-      n.cut = list_select<kThreads>(h, listed, 0ull, static_cast<unsigned long long>(top_k - 1), whole_row(), scratch);
+      n.cut = list_select<kThreads>(h, listed, 0ull, static_cast<unsigned long long>(top_k - 1), whole_row());
       const auto sum_kept = [&]() {
         unsigned long long zfix = 0ull;
         for (int j = threadIdx.x; j < listed; j += kThreads)
@@ -583,13 +698,13 @@ __device__ __forceinline__ RowNorm block_normalise(const T* __restrict__ row, in
           mass += w;
         }
         if (block_sum<kThreads>(mass, scratch) > limit_p) {
-          n.cut = list_select<kThreads>(h, listed, 0ull, limit_p, outer, scratch);
+          n.cut = list_select<kThreads>(h, listed, 0ull, limit_p, outer);
           n.z = sum_kept();
         }
       }
       return n;
     }
-    n.cut = bucket_select<T, kThreads, false>(row, vocab, temperature, n.m, 0.0f, whole_row(),
+    n.cut = bucket_select<T, kThreads, false>(row, vocab, temperature, n.m, 0.0f, own, whole_row(),
                                               static_cast<unsigned long long>(top_k - 1), scratch, h);
     n.z = block_cut_sum<T, kThreads>(row, vocab, temperature, n.m, n.cut, scratch);
   } else {
@@ -597,7 +712,7 @@ __device__ __forceinline__ RowNorm block_normalise(const T* __restrict__ row, in
   }
   if (use_p) {
     const Cut outer = n.cut;
-    n.cut = bucket_select<T, kThreads, true>(row, vocab, temperature, n.m, RLT_DIV(1.0f, n.z), outer, limit_p, scratch, h);
+    n.cut = bucket_select<T, kThreads, true>(row, vocab, temperature, n.m, RLT_DIV(1.0f, n.z), own, outer, limit_p, scratch, h);
     if (n.cut.key != outer.key || n.cut.limit != outer.limit)
       n.z = block_cut_sum<T, kThreads>(row, vocab, temperature, n.m, n.cut, scratch);
   }
@@ -620,8 +735,8 @@ __device__ __forceinline__ float prob_at(const T* row, int v, float temperature,
 // Inverse-CDF draw over fixed-point weights in ascending token index, p[v] (plain) or max(p[v] - q[v], 0) (residual) in the
 // division-free form of rlt_canonical.h; -1 if the mass is zero.  A warp owns a run of tokens and reads it 128 tokens at a time, four
 // per lane; the warp in whose run the threshold falls goes over its run once more.  Tokens outside p's support weigh nothing and are
-// dismissed by one comparison, q is read where p has mass only.  (A run of tokens per THREAD, the earlier split, read a line per
-// lane: a residual draw from two rows of 49 152 took 74 us, this 56.)
+// dismissed by one comparison, q is read where p has mass only.  128 requests that draw from the residual of two rows of 49 152, or from a
+// bonus row: 55 us (74 us where a thread, not a warp, has a run of tokens, whose every load is a line of its own).
 template <typename T, int kThreads>
 __device__ __forceinline__ int block_draw(const T* __restrict__ prow, const RowNorm& pn,
                                           const T* __restrict__ qrow, const RowNorm& qn, bool residual,
@@ -660,10 +775,10 @@ __device__ __forceinline__ int block_draw(const T* __restrict__ prow, const RowN
     }
     return sum;
   };
-  unsigned long long w[kLane], local = 0ull;
+  unsigned long long w[kLane] = {0ull, 0ull, 0ull, 0ull}, own = 0ull;
 #pragma unroll 2
-  for (int v = begin + lane * kLane; v < end; v += kStep) local += weigh(v, w);
-  local = warp_sum(local);
+  for (int v = begin + lane * kLane; v < end; v += kStep) own += weigh(v, w);
+  const unsigned long long local = warp_sum(own);
   __syncthreads();
   if (lane == 0) scratch[warp] = local;
   if (threadIdx.x == 0) *token_slot = -1;
@@ -678,7 +793,7 @@ __device__ __forceinline__ int block_draw(const T* __restrict__ prow, const RowN
     const unsigned long long threshold = rlt_draw_threshold(u, total);
     if (before <= threshold && threshold < before + local) {           // one warp
       for (int at = begin; at < end; at += kStep) {
-        const unsigned long long sum = weigh(at + lane * kLane, w);
+        const unsigned long long sum = run == kStep ? own : weigh(at + lane * kLane, w);   // (a run of one step is still at hand)
         unsigned long long upto = sum;
 #pragma unroll
         for (int x = 1; x < 32; x <<= 1) {
