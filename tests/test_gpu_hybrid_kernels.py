@@ -177,10 +177,11 @@ def test_block_epilogue(dtype, kv_heads, dim, vdim, ff, kind):
         close(out[:, 8:], plain.gelu(x) if kind == "gelu" else plain.gelu_tanh(x), dtype)
 
 
-@pytest.mark.parametrize("rows", [511, 512, 513, 515, 1030])
+@pytest.mark.parametrize("rows", [511, 512, 513, 515, 1030, 21399, 21400, 22309, 22311, 22313])
 @pytest.mark.parametrize("kv_heads,dim,ff", [(2, 64, 136), (3, 5, 17)])
 def test_block_epilogue_of_a_prompt(rows, kv_heads, dim, ff):
-    """Several rows per thread: a last thread with some of them, pages and padding rows among them."""
+    """One row per thread and, from 2^20 accesses on (49 a row of the first widths, 47 of the second), several: a last thread with some of them,
+    pages and padding rows among them."""
     g = torch.Generator().manual_seed(rows)
     width, pages = kv_heads * dim, -(-rows // BLOCK)
     proj = torch.randn(rows, 2 * width + ff, generator=g).bfloat16().cuda()

@@ -303,7 +303,11 @@ gated_norm_parts_kernel(const T* __restrict__ y, int64_t y_stride, const T* __re
   }
 }
 
-constexpr int kRowsPerThread = 4, kManyRows = 512;    // block_epilogue_kernel
+// block_epilogue_kernel: four rows per thread from 2^20 accesses on.  One row / four rows per thread, us, bf16: 1024 keys and values each beside
+// 8448 gelu columns 6.85 / 6.95 for 512 rows, 9.12 / 8.90 for 768, 15.5 / 14.2 for 1536, 40.7 / 35.0 for 4096; 2048 and no activations 5.31 / 5.52
+// for 1024, 8.88 / 8.09 for 2048; 512 and 2816 columns 8.38 / 8.79 for 2048, 14.3 / 13.5 for 4096; 256 and 704 columns 5.60 / 6.28 for 3072.
+constexpr int kRowsPerThread = 4;
+constexpr int64_t kManyItems = 1 << 20;
 constexpr int kMaxPer = 12;   // accesses of 4 elements per thread of a residual row
 constexpr size_t kMaxRowBytes = 48u * 1024u;   // a staged row of fp32 values
 
@@ -380,7 +384,7 @@ extern "C" RLT_API int rlt_block_epilogue(const void* proj, int64_t proj_stride,
            whole(v_block_stride) && whole(v_token_stride) && aligned16(key_cache) && aligned16(value_cache);
   if (act_width > 0) wide = wide && whole(act_col) && whole(act_width) && whole(out_stride) && whole(out_col) && aligned16(out);
   const int items = (k_width + v_width + act_width) / (wide ? vec : 1);
-  const bool many = rows >= kManyRows;          // a prompt's: enough CTAs with several rows each
+  const bool many = static_cast<int64_t>(rows) * items >= kManyItems;          // a prompt's: enough CTAs with several rows each
   const int per = many ? kRowsPerThread : 1;
   const dim3 grid(static_cast<unsigned>((rows + per - 1) / per), static_cast<unsigned>((items + kThreads - 1) / kThreads));
   cudaStream_t s = static_cast<cudaStream_t>(stream);
