@@ -754,7 +754,9 @@ RLT_API int rlt_delta_scan(const void* q, const void* k, const void* v, int64_t 
  * sequence `short_sequences` on counted from there, starts, lengths, slots [sequences], and page tables [planes][sequences][width].  records
  * [portions][5 + 2 planes]: address of the portion's int64 tokens, their number, tokens stored before, slot, the last of them (-1: none), then per
  * plane the address of the int32 page ids and their number (those beyond width are left out, the rest of a table row is zero).  Sequences behind
- * the portions are padding: one row, row_seq -1, previous -1, length 0, dummy_slot.  RLT_ERR_INVALID where `rows` is not what they add up to. */
+ * the portions are padding: one row, row_seq -1, previous -1, length 0, dummy_slot.  The tokens' words must be 8-byte aligned.  RLT_ERR_INVALID, with
+ * nothing written, where `rows` is not what they add up to, a portion has no tokens, negative positions or positions beyond 32 bits, or a number of pages is
+ * negative or has no address. */
 RLT_API int rlt_step_metadata(int32_t* words, const int64_t* at, const int64_t* records, int portions, int sequences, int planes, int width,
                       int short_sequences, int64_t rows, int64_t dummy_slot);
 

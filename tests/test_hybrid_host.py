@@ -217,6 +217,25 @@ def test_step_metadata_is_what_a_loop_over_the_tokens_says(counts, starts, paddi
     assert v["tables"][0].tolist() == [(cache.pages(i) + [0] * 4)[:4] for i in range(len(counts))] + [[0] * 4] * padding
 
 
+@pytest.mark.parametrize("place, value", [(0, 0), (1, 0), (1, -3), (1, 5), (2, -1), (2, 2 ** 31 - 3), (2, 2 ** 31), (2, 2 ** 62), (6, -8), (6, -2 ** 62), (5, 0), (8, -1), (7, 0)])
+def test_step_metadata_refuses_records_that_lead_outside(place, value):
+    """A portion of three tokens behind four stored ones, two pages on each of two planes; one word of its record is spoilt."""
+    layout = engine_module._Layout(3, 1, 2, 4, 1)
+    words = torch.full((layout.size + 16,), 77, dtype=torch.int32)
+    tokens, pages = torch.tensor([5, 6, 7]), torch.tensor([1, 2], dtype=torch.int32)
+    records = torch.tensor([tokens.data_ptr(), 3, 4, 0, 9, pages.data_ptr(), 2, pages.data_ptr(), 2])
+    at = torch.tensor([8 + where.start for where in layout.at.values()])
+    fill = lambda at: rlt._capi.load().rlt_step_metadata(words.data_ptr(), at.data_ptr(), records.data_ptr(), 1, 1, 2, 4, 1, 3, 9)
+    assert fill(at) == rlt._capi.OK
+    assert words[:8].eq(77).all() and words[8 + layout.size:].eq(77).all()
+    assert layout.views(words[8:8 + layout.size])["tables"].tolist() == [[[1, 2, 0, 0]], [[1, 2, 0, 0]]]
+    words.fill_(77)
+    for bad in (at + torch.eye(10, dtype=torch.int64)[0], at - 100):       # tokens between two 8-byte words; offsets in front of the words
+        assert fill(bad) == rlt._capi.ERR_INVALID and words.eq(77).all()
+    records[place] = value
+    assert fill(at) == rlt._capi.ERR_INVALID and words.eq(77).all()
+
+
 def test_tokens_of_other_kinds_are_taken_as_whole_numbers(counting_engine):
     engine, tokens = counting_engine(), prompt(3, 20, 53)
     for name, other in enumerate((tuple(tokens), [float(t) for t in tokens], [torch.tensor(t) for t in tokens])):

@@ -14,12 +14,19 @@ extern "C" RLT_API int rlt_step_metadata(int32_t* words, const int64_t* at, cons
   RLT_REQUIRE(portions >= 0 && portions <= sequences && planes >= 1 && width >= 0 && short_sequences >= 0 && short_sequences <= sequences,
               "step_metadata: bad counts");
   const int record = 5 + 2 * planes;
+  RLT_REQUIRE(rows >= 0 && rows <= 0x7fffffff, "step_metadata: bad counts");
+  for (int i = kTokens; i <= kTables; ++i) RLT_REQUIRE(at[i] >= 0, "step_metadata: an offset in front of the words");
+  RLT_REQUIRE((reinterpret_cast<uintptr_t>(words + at[kTokens]) & 7u) == 0, "step_metadata: tokens need 8-byte alignment");
   int64_t needed = sequences - portions;
   for (int i = 0; i < portions; ++i) {
-    RLT_REQUIRE(records[static_cast<int64_t>(i) * record + 1] >= 1, "step_metadata: a portion without tokens");
-    needed += records[static_cast<int64_t>(i) * record + 1];
+    const int64_t* r = records + static_cast<int64_t>(i) * record;
+    RLT_REQUIRE(r[0] != 0 && r[1] >= 1, "step_metadata: a portion without tokens");
+    RLT_REQUIRE(r[1] <= rows && r[2] >= 0 && r[2] <= 0x7fffffff - r[1], "step_metadata: positions beyond 32 bits");
+    for (int plane = 0; plane < planes; ++plane)
+      RLT_REQUIRE(r[6 + 2 * plane] >= 0 && (r[6 + 2 * plane] == 0 || r[5 + 2 * plane] != 0), "step_metadata: a page table without pages");
+    needed += r[1];
   }
-  RLT_REQUIRE(needed == rows && rows <= 0x7fffffff, "step_metadata: the rows are not the portions' and the padding's");
+  RLT_REQUIRE(needed == rows, "step_metadata: the rows are not the portions' and the padding's");
   int64_t* tokens = reinterpret_cast<int64_t*>(words + at[kTokens]);
   int32_t *positions = words + at[kPositions], *row_seq = words + at[kRowSeq], *previous = words + at[kPrevious], *cu = words + at[kCu];
   int32_t row = 0;

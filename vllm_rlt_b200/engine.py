@@ -257,7 +257,8 @@ class Engine:
             kept.append(tokens)
             records.extend((tokens.buffer_info()[0], len(tokens), cache.length(p.name), cache.slot(p.name), int(cache.last_token(p.name))))
             for plane in range(layout.planes):
-                records.extend(cache.page_words(p.name, plane).buffer_info())
+                kept.append(cache.page_words(p.name, plane))    # (alive until the call returns, whoever gives the sequence back meanwhile)
+                records.extend(kept[-1].buffer_info())
         at = array("q", [where.start for where in layout.at.values()])
         _capi.check(_capi.load().rlt_step_metadata(host.data_ptr(), at.buffer_info()[0], records.buffer_info()[0], len(portions), layout.sequences,
                                                    layout.planes, layout.width, layout.short, layout.rows, cache.dummy_slot), "step")
