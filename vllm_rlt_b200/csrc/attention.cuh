@@ -92,36 +92,35 @@ __device__ __forceinline__ float softmax_scale(float m, float l, float sink) {
   return f / fmaf(l, f, 1.0f);
 }
 
+// Tokens that a row of the block table can address.
+__device__ __forceinline__ int table_capacity(const AttentionArgs& a) {
+  const int64_t tokens = static_cast<int64_t>(a.table_width) * a.block_size;
+  return tokens > 0x7fffffff ? 0x7fffffff : static_cast<int>(tokens);
+}
+// Keys that query row `row` sees, a row of the sequence that owns rows first .. end - 1 and has `context` keys with them.
+__device__ __forceinline__ int packed_keys(int context, int first, int end, int row) { return context - (end - first) + (row - first) + 1; }
+// The lengths live on the device (graph replays change them without the host seeing them), so a length beyond what the row's table can
+// address is clamped: no kernel ever indexes a table row past its width.
+__device__ __forceinline__ int clamped_keys(int keys, int capacity) { return max(min(keys, capacity), 0); }
+
 // Table row and number of visible keys of query row `row`.
 // Unpacked: its own table row and context length.  Packed: the sequence s that contains
 // the row, and context_lengths[s] - n_s + i + 1 for its i-th of n_s rows.
-// The lengths live on the device (graph replays change them without the host seeing them), so
-// a length beyond what the row's table can address (table_width * block_size tokens) is
-// clamped here: no kernel ever indexes a table row past its width.  `*clamped` (optional) is
-// set when that happened, so that the caller can report it.
-__device__ __forceinline__ void resolve_row(const AttentionArgs& a, int row, int* table_row, int* len,
-                                            bool* clamped = nullptr) {
-  const int64_t capacity64 = static_cast<int64_t>(a.table_width) * a.block_size;
-  const int capacity = capacity64 > 0x7fffffff ? 0x7fffffff : static_cast<int>(capacity64);
-  int n;
+__device__ __forceinline__ void resolve_row(const AttentionArgs& a, int row, int* table_row, int* len) {
+  int keys;
   if (a.cu_seqlens_q == nullptr) {
     *table_row = row;
-    n = a.context_lengths[row];
+    keys = a.context_lengths[row];
   } else {
     int lo = 0, hi = a.table_rows - 1;  // last s with cu[s] <= row
     while (lo < hi) {
       int mid = (lo + hi + 1) >> 1;
       if (a.cu_seqlens_q[mid] <= row) lo = mid; else hi = mid - 1;
     }
-    const int first = a.cu_seqlens_q[lo], count = a.cu_seqlens_q[lo + 1] - first;
     *table_row = lo;
-    n = a.context_lengths[lo] - count + (row - first) + 1;
+    keys = packed_keys(a.context_lengths[lo], a.cu_seqlens_q[lo], a.cu_seqlens_q[lo + 1], row);
   }
-  if (n > capacity) {
-    n = capacity;
-    if (clamped != nullptr) *clamped = true;
-  }
-  *len = n > 0 ? n : 0;
+  *len = clamped_keys(keys, table_capacity(a));
 }
 
 // attention_generic.cu: any shape, one CTA per (row, head).

@@ -196,19 +196,17 @@ plan_kernel(AttentionArgs a, Workspace ws, int cap) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int row = blockIdx.x * (kPlanThreads / 32) + warp;
   if (row < a.rows) {
-    // the row as resolve_row has it; lengths beyond the table are clamped
-    const int64_t capacity64 = static_cast<int64_t>(a.table_width) * a.block_size;
-    const int capacity = capacity64 > 0x7fffffff ? 0x7fffffff : static_cast<int>(capacity64);
-    int table_row = row, first = row, seen;
+    const int capacity = table_capacity(a);
+    int table_row = row, first = row, seen;       // as resolve_row has them, the sequence found by the whole warp
     if (a.cu_seqlens_q == nullptr) {
       seen = a.context_lengths[row];
     } else {
       table_row = sequence_of(a.cu_seqlens_q, a.table_rows, row);
       first = a.cu_seqlens_q[table_row];
-      seen = a.context_lengths[table_row] - (a.cu_seqlens_q[table_row + 1] - first) + (row - first) + 1;
+      seen = packed_keys(a.context_lengths[table_row], first, a.cu_seqlens_q[table_row + 1], row);
     }
     if (seen > capacity && lane == 0) atomicOr(&ws.header->error, kErrorLengthClamped);
-    const int len = max(min(seen, capacity), 0);
+    const int len = clamped_keys(seen, capacity);
     int link = 0;
     if (len > 0 && row > 0) {
       const bool packed = a.cu_seqlens_q != nullptr;
