@@ -635,31 +635,40 @@ __device__ __forceinline__ Cut bucket_select(const T* __restrict__ row, int voca
   return cut_of_ties(at.key, at.ties, at.each, at.before);
 }
 
-// max, support and normaliser of the distribution Sampler.probabilities builds for one row
-// (vllm_rlt/worker/sampler.py:37-55): softmax(row / T) restricted to top-k, then to top-p.
-// top_k <= 0 or >= vocab and top_p >= 1 switch the filters off.
-// Division by a positive temperature is monotonic, so max_v (x_v / T) == (max_v x_v) / T exactly: the first pass is a plain
-// maximum over the raw logits, one division at the end.
+// max of row / temperature, and the thread's own largest raw logit.  Division by a positive temperature is monotonic, so
+// max_v (x_v / T) == (max_v x_v) / T exactly: the pass is a plain maximum over the raw logits, one division at the end.
 template <typename T, int kThreads>
-__device__ __forceinline__ RowNorm block_normalise(const T* __restrict__ row, int vocab, float temperature,
-                                                   int top_k, float top_p, unsigned long long* scratch,
-                                                   SelectScratch& h) {
-  const bool use_k = top_k > 0 && top_k < vocab, use_p = top_p < 1.0f;
-  float own = -INFINITY;
+__device__ __forceinline__ RowNorm block_row_max(const T* __restrict__ row, int vocab, float temperature, unsigned long long* scratch,
+                                                 float* own) {
+  float largest = -INFINITY;
   bool nan = false;
   for_row<T, kThreads>(row, vocab, [&](float x, int) {
-    own = fmaxf(own, x);
+    largest = fmaxf(largest, x);
     nan |= x != x;
   });
-  const uint32_t own_key = rlt_order_key(own);
-  const uint32_t top = __reduce_max_sync(0xffffffffu, nan ? 0xffffffffu : own_key);
+  *own = largest;
+  const uint32_t top = __reduce_max_sync(0xffffffffu, nan ? 0xffffffffu : rlt_order_key(largest));
   RowNorm n;
   const uint32_t best = static_cast<uint32_t>(block_max<kThreads>(top, scratch));
   n.m = best == 0xffffffffu ? NAN : RLT_DIV(key_value(best), temperature);
   n.ok = n.m == n.m && n.m != INFINITY && n.m != -INFINITY;
   n.z = 0.0f;
   n.cut = whole_row();
+  return n;
+}
+
+// max, support and normaliser of the distribution Sampler.probabilities builds for one row
+// (vllm_rlt/worker/sampler.py:37-55): softmax(row / T) restricted to top-k, then to top-p.
+// top_k <= 0 or >= vocab and top_p >= 1 switch the filters off.
+template <typename T, int kThreads>
+__device__ __forceinline__ RowNorm block_normalise(const T* __restrict__ row, int vocab, float temperature,
+                                                   int top_k, float top_p, unsigned long long* scratch,
+                                                   SelectScratch& h) {
+  const bool use_k = top_k > 0 && top_k < vocab, use_p = top_p < 1.0f;
+  float own;
+  RowNorm n = block_row_max<T, kThreads>(row, vocab, temperature, scratch, &own);
   if (!n.ok) return n;
+  const uint32_t own_key = rlt_order_key(own);
   const unsigned long long limit_p = rlt_top_p_limit(top_p);
   if (use_k) {
     int listed = kCandidates + 1;
@@ -716,6 +725,15 @@ __device__ __forceinline__ RowNorm block_normalise(const T* __restrict__ row, in
     if (n.cut.key != outer.key || n.cut.limit != outer.limit)
       n.z = block_cut_sum<T, kThreads>(row, vocab, temperature, n.m, n.cut, scratch);
   }
+  return n;
+}
+
+// The same without filters, for kernels that keep their registers free of them.
+template <typename T, int kThreads>
+__device__ __forceinline__ RowNorm block_normalise_plain(const T* __restrict__ row, int vocab, float temperature, unsigned long long* scratch) {
+  float own;
+  RowNorm n = block_row_max<T, kThreads>(row, vocab, temperature, scratch, &own);
+  if (n.ok) n.z = block_full_sum<T, kThreads>(row, vocab, temperature, n.m, scratch);
   return n;
 }
 
@@ -893,14 +911,13 @@ __device__ __forceinline__ int request_of_row(const int32_t* cu_rows, int n, int
   return lo;
 }
 
-template <typename T, int kThreads>
+template <typename T, int kThreads, bool kFilters>
 __global__ void __launch_bounds__(kThreads, 3)
 row_stats_kernel(const T* __restrict__ target_logits, const T* __restrict__ draft_logits, int64_t row_stride,
                  int vocab, const int32_t* __restrict__ cu_rows, int n, const int32_t* __restrict__ row_counts,
                  const int64_t* __restrict__ tokens, int tokens_width, const float* __restrict__ temperature,
                  const int32_t* __restrict__ top_k, const float* __restrict__ top_p, RowStats* __restrict__ stats) {
   __shared__ unsigned long long scratch[32];
-  __shared__ SelectScratch select;
   const int row = blockIdx.x, side = blockIdx.y;  // side 0: target, 1: draft
   const int i = request_of_row(cu_rows, n, row);
   int first, span;
@@ -915,8 +932,13 @@ row_stats_kernel(const T* __restrict__ target_logits, const T* __restrict__ draf
   } else {
     if (side == 1 && j == count - 1) return;  // the bonus row has no draft distribution
     const T* logits = (side == 0 ? target_logits : draft_logits) + static_cast<int64_t>(row) * row_stride;
-    const RowNorm norm = block_normalise<T, kThreads>(logits, vocab, temp, top_k ? top_k[i] : -1, top_p ? top_p[i] : 1.0f, scratch,
-                                                      select);
+    RowNorm norm;
+    if constexpr (kFilters) {
+      __shared__ SelectScratch select;
+      norm = block_normalise<T, kThreads>(logits, vocab, temp, top_k ? top_k[i] : -1, top_p ? top_p[i] : 1.0f, scratch, select);
+    } else {
+      norm = block_normalise_plain<T, kThreads>(logits, vocab, temp, scratch);
+    }
     const int64_t d = j < count - 1 ? tokens[static_cast<int64_t>(i) * tokens_width + j + 1] : -1;
     out.m = norm.m;
     out.z = norm.z;
@@ -1141,10 +1163,12 @@ extern "C" RLT_API int rlt_accept_rejection(const void* target_logits, const voi
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   RowStats* stats = static_cast<RowStats*>(workspace);
-  RLT_DISPATCH_DTYPE(dtype, T, (row_stats_kernel<T, kStatsThreads><<<dim3(rows, 2), kStatsThreads, 0, s>>>(
-                                   static_cast<const T*>(target_logits), static_cast<const T*>(draft_logits),
-                                   row_stride, vocab, cu_rows, n, row_counts, tokens, tokens_width, temperature,
-                                   top_k, top_p, stats)));
+  const bool filters = top_k != nullptr || top_p != nullptr;
+  RLT_DISPATCH_DTYPE(dtype, T, {
+    auto kernel = filters ? row_stats_kernel<T, kStatsThreads, true> : row_stats_kernel<T, kStatsThreads, false>;
+    kernel<<<dim3(rows, 2), kStatsThreads, 0, s>>>(static_cast<const T*>(target_logits), static_cast<const T*>(draft_logits), row_stride, vocab,
+                                                   cu_rows, n, row_counts, tokens, tokens_width, temperature, top_k, top_p, stats);
+  });
   status = launch_status("row_stats_kernel");
   if (status != RLT_OK) return status;
   RLT_DISPATCH_DTYPE(dtype, T, (decide_kernel<T><<<n, kSampleThreads, 0, s>>>(

@@ -36,7 +36,7 @@ struct ConvArgs {
 // columns (839 MB) 201 us; with a bound checked per token, spilled registers and two rows of activations ahead, 116 and 236 us.
 // kTaps 0: any number of taps, inputs re-read (from L1) for every output, one channel per thread.
 template <typename T, int kTaps, int kVec, int kActVec>
-__global__ void __launch_bounds__(kThreads, kTaps > 0 ? 6 : 8)
+__global__ void __launch_bounds__(kThreads, kTaps > 0 ? 6 : kActVec > 1 ? 9 : 8)
 causal_conv_kernel(ConvArgs a) {
   const int seq = blockIdx.z, first = blockIdx.y * kTile;
   const int row0 = a.cu[seq], n = a.cu[seq + 1] - row0;
