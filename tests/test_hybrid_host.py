@@ -247,6 +247,16 @@ def test_tokens_of_other_kinds_are_taken_as_whole_numbers(counting_engine):
                 engine.step([dict(name="a", tokens=[1] * (length - 1) + [bad])])
 
 
+@pytest.mark.parametrize("tokens", [iter([1, 2]), {1, 2}, {1: 2}, (t for t in [1] * 20)])
+def test_tokens_that_are_no_sequence_are_refused_and_change_nothing(counting_engine, tokens):
+    engine = counting_engine()
+    before = engine.cache.free_slots, engine.cache.free_pages
+    with pytest.raises((TypeError, KeyError)):
+        engine.step([dict(name="a", tokens=tokens)])
+    assert "a" not in engine.cache and (engine.cache.free_slots, engine.cache.free_pages) == before
+    assert engine.step([dict(name="a", tokens=range(1, 20), want=[18])]).shape == (1, 53)
+
+
 def test_a_step_that_does_not_fit_changes_nothing(counting_engine):
     engine = counting_engine(max_tokens=64, max_sequences=2)
     engine.step([dict(name="a", tokens=[1] * 40)])

@@ -39,6 +39,7 @@ class _Portion:
 
     def __init__(self, entry: StepEntry, vocab: int):
         self.name, tokens = entry.name, entry.tokens
+        tokens[:0]                                         # a sequence: an iterator would be used up here, a set has no order
         try:
             self.tokens = array("q", tokens if type(tokens) in (list, tuple) else list(tokens))
         except (TypeError, OverflowError):                 # numbers of other kinds, or beyond any vocabulary
