@@ -227,12 +227,13 @@ def test_filters_where_a_selection_changes_its_way_match_oracle_bit_for_bit(voca
         assert torch.equal(tokens.cpu(), oracle.sample_rows(logits.contiguous(), temperature, uniforms, top_k, top_p)[0])
 
 
-@pytest.mark.parametrize("vocab,dtype", [(49152, torch.float32), (20001, torch.bfloat16), (3000, torch.float32)])
+@pytest.mark.parametrize("vocab,dtype", [(49152, torch.float32), (20001, torch.bfloat16), (3000, torch.float32), (2050, torch.float16),
+                                         (2048, torch.float32), (2047, torch.float32), (129, torch.float32), (128, torch.bfloat16), (127, torch.float32)])
 def test_filters_of_rows_that_a_histogram_has_to_divide_again(vocab, dtype):
     """Rows whose bulk is narrow beside its distance from a peak or from masked tokens, bands of their own, ties in the thousands and values next
-    to each other: the steps of the first histogram, of the next ones, and what no step tells apart."""
+    to each other: the steps of the first histogram, of the next ones, and what no step tells apart; rows that just fit a list, or one warp."""
     g = torch.Generator().manual_seed(vocab)
-    x = torch.randn(10, vocab, generator=g)
+    x = torch.randn(12, vocab, generator=g)
     x[0] *= 1e-3
     x[1] = x[1] * 1e-3 - 8
     x[1, 7] = 0.0                                       # the bulk in one step of the first histogram
@@ -246,14 +247,17 @@ def test_filters_of_rows_that_a_histogram_has_to_divide_again(vocab, dtype):
     x[8] *= 300
     x[8, 5] = 3e4
     x[9, vocab // 2:] = float("-inf")
+    for row, peak, spread in ((10, 1e4, (9.0, 4e-3, 1e-9)), (11, 8.0, (7e-3, 3e-6, 1e-12))):   # a bulk that three histograms leave in one step:
+        x[row] *= spread[-1]                            # each is stretched by a pair of tokens around it
+        x[row, :5] = torch.tensor([peak, spread[0], -spread[0], spread[1], -spread[1]])
     logits = x.to(dtype)
-    cuda, ones = logits.cuda(), torch.ones(10)
+    cuda, ones = logits.cuda(), torch.ones(12)
     for top_k, top_p, temperature in ((-1, 0.95, 0.8), (-1, 0.3, 1.0), (vocab - 3, 1.0, 1.0), (1500, 0.5, 1.0), (2500, 0.9999, 1e-3), (50, 0.95, 1e3), (300, 0.7, 1.0)):
-        k, p, t = torch.full((10,), top_k, dtype=torch.int32), ones * top_p, ones * temperature
+        k, p, t = torch.full((12,), top_k, dtype=torch.int32), ones * top_p, ones * temperature
         want = _oracle_probabilities(logits, t, k, p)
         got, status = rlt.probabilities(cuda, t.cuda(), k.cuda(), p.cuda())
         assert not status.any()
-        assert torch.equal(got.cpu(), want), (top_k, top_p, [r for r in range(10) if not torch.equal(got[r].cpu(), want[r])])
+        assert torch.equal(got.cpu(), want), (top_k, top_p, [r for r in range(12) if not torch.equal(got[r].cpu(), want[r])])
 
 
 def test_probabilities_reject_greedy_and_bad_rows():

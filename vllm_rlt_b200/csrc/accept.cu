@@ -314,7 +314,7 @@ __device__ __forceinline__ void list_token(SelectScratch& h, uint32_t key, int i
 }
 
 // Adds to a bucket by atomics on its two words, the low one's carry going into the high one: 32-bit adds are done by the memory itself, a 64-bit
-// one retries for as long as other lanes get in between, which takes 40 times as long where the tokens of a row share a bucket.
+// one retries for as long as other lanes get in between (top-p of a row of 49 152 equal logits: 206 us, with 64-bit atomics 2144).
 __device__ __forceinline__ void bucket_add(SelectScratch& h, int bucket, unsigned long long w) {
   unsigned* word = reinterpret_cast<unsigned*>(&h.bucket[bucket]);
   const unsigned low = static_cast<unsigned>(w), before = atomicAdd(word, low);

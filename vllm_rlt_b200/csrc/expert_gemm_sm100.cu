@@ -304,6 +304,10 @@ int launch_expert_gemm_sm100(const ExpertGemm& g, cudaStream_t stream) {
   DeviceInfo info;
   const int status = current_device_info(&info);
   if (status != RLT_OK) return status;
+  // Rows of 128 in single CTAs / of 256 in pairs, us: 64 experts of 704 -> 2048 with 64 rows each 37 / 40, 96: 40 / 42, 128: 42 / 44, 160: 58 / 48,
+  // and of unequal numbers, which routing gives, 64: 38 / 40, 96: 42 / 42, 112: 46 / 44, 128: 49 / 47, 192: 61 / 53; 2048 -> 1408 unequal 96: 73 / 77,
+  // 112: 79 / 77, 128: 87 / 81.  (8 experts of 4096 -> 2816 take pairs from 16 rows on, 47 / 46; at 96 50 / 47.)  Rows of 32 / of 128 at 24 rows: 63 / 64
+  // and 70 / 64 unequal, at 48 88 / 66.  One block of outputs, 64 experts of 2048 -> 128: single CTAs 16 / pairs 16 for 128 rows, 35 / 37 for 512.
   const int64_t average = g.rows / g.experts;
   if (average <= 24) return launch<32, 1>(g, info.sm_count, stream);
   if (average <= 96 || g.out <= kOutputs) return launch<128, 1>(g, info.sm_count, stream);   // one block of outputs: nothing for a second CTA

@@ -134,8 +134,10 @@ sandwich_norm_vec_kernel(const T* __restrict__ x, const T* __restrict__ weight, 
 
 // The same with a warp per row: eight 16-byte vectors of the row and of the residual in a lane's registers, no barriers, so the warps of an
 // SM drift apart and some are always loading.  For the rows of a prompt; a decoding step's few rows are quicker spread over a CTA each.
-// 7402 rows of 2048 in bf16 with residual and both norms: 36.4 -> 31.1 us (121 MB, 18.5 us; sums in double take the rest).  Few rows stay with
-// a CTA each: a step of 8 rows takes 2.5 us that way.
+// A CTA per row / a warp per row, us, 2048 bf16 with residual and both norms: 3.8 / 6.6 for 256 rows, 6.3 / 7.2 for 768, 7.4 / 7.3 for 1024, 10.7 /
+// 9.4 for 1536, 12.9 / 13.7 for 2048 (a second wave of few CTAs), 15.2 / 14.3 for 2560, 22.3 / 20.4 for 4096, 38.6 / 36.3 for 7402, 81 / 69 for
+// 16384; one norm alone: 4.5 / 5.0 for 768, 5.2 / 5.0 for 1024, 8.7 / 8.1 for 2048, 25.9 / 18.1 for 7402; fp16 and fp32 gain more.  So from 1024
+// rows on.  In a prompt step of the looped model, which runs at the power cap, the two are equal (13.56 and 13.62 ms, medians of twelve turns).
 template <typename T>
 __global__ void __launch_bounds__(kRowWarps * 32)
 sandwich_norm_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight, const T* residual, T* sum_out,
