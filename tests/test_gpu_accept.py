@@ -260,6 +260,28 @@ def test_filters_of_rows_that_a_histogram_has_to_divide_again(vocab, dtype):
         assert torch.equal(got.cpu(), want), (top_k, top_p, [r for r in range(12) if not torch.equal(got[r].cpu(), want[r])])
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("vocab", [1, 3, 17, 513, 4101, 4127])
+def test_rows_of_any_alignment_are_read_alike(vocab, dtype):
+    """Every offset from a 16-byte boundary: elements in front of the first whole vector and behind the last, runs of a draw that start inside one."""
+    per, g = 16 // dtype.itemsize, torch.Generator().manual_seed(vocab)
+    rows = torch.randn(per, vocab, generator=g).mul(2).to(dtype)
+    width = -(-(vocab + per) // per) * per
+    cuda, t = torch.empty(per, width, dtype=dtype, device="cuda"), torch.full((1,), 0.9)
+    for shift in range(per):
+        cuda.fill_(float("nan"))                           # what a read beyond the row would find
+        cuda[:, shift:shift + vocab] = rows.cuda()
+        view = cuda[:, shift:shift + vocab]
+        for r in range(0, per, 3):
+            one, u = view[r:r + 1], torch.rand(1, generator=g)
+            for top_k, top_p in ((-1, 1.0), (5, 0.9), (-1, 0.8)):
+                k, p = torch.tensor([top_k], dtype=torch.int32), torch.tensor([top_p])
+                got, status = rlt.probabilities(one, t.cuda(), k.cuda(), p.cuda())
+                assert not status.any() and torch.equal(got.cpu(), _oracle_probabilities(rows[r:r + 1], t, k, p)), (shift, r, top_k, top_p)
+                tokens, _ = rlt.sample_rows(one, t.cuda(), u.cuda(), k.cuda(), p.cuda())
+                assert torch.equal(tokens.cpu(), oracle.sample_rows(rows[r:r + 1].contiguous(), t, u, k, p)[0])
+
+
 def test_probabilities_reject_greedy_and_bad_rows():
     logits = torch.randn(3, 64)
     logits[2, 5] = float("nan")
